@@ -2,8 +2,8 @@
 // estimate: the two scheduled routines of AsterX outside the RHS and
 // post-step groups that read the evolved state every step.
 //
-//   k_tmunu<ORDER, ZVEC>   AsterX_Tmunu (AsterX/src/tmunu.cxx:19-178): the
-//                          cell-centred primitives interpolated to each
+//   k_tmunu2<ZVEC>,        AsterX_Tmunu (AsterX/src/tmunu.cxx:19-178): the
+//   k_tmunu4<ZVEC>         cell-centred primitives interpolated to each
 //                          interior vertex (AsterUtils/src/aster_interp.hxx:
 //                          97-148, order 2 or 4), T_{mu nu} of the ideal
 //                          MHD fluid added to eTtt .. eTzz
@@ -11,8 +11,8 @@
 //                          estimate_error.cxx:70-144) with the indicators of
 //                          AsterX/src/estimate_error.hxx:14-86
 //
-// Both are HBM-bound point loops (one thread per point, rows of 128 along
-// x, neighbours from L1/L2).  This file is compiled without multiply-add
+// k_tmunu2 and k_regrid_error are HBM-bound point loops (one thread per point,
+// rows of 128 along x, neighbours from L1/L2).  This file is compiled without multiply-add
 // contraction and keeps the reference's operation order (sums from left to
 // right, products left-associated as written), so the results are the
 // reference's bits: IEEE division and square root round the same on both.
@@ -29,7 +29,7 @@ namespace {
 // ---------------------------------------------------------------------------
 struct TmunuArgs {
   BoxDev b;
-  const double *rho, *eps, *press, *v[3], *B[3];
+  const double *f[9]; // rho, eps, press, B^x..B^z, v^x..v^z or z^x..z^z
   const double *g[6], *alp, *beta[3];
   double *eT[10];
 };
@@ -48,70 +48,11 @@ AXB_D double c2v2(const double *__restrict__ f, long long I, long long sy, long 
   return s / 8.0;
 }
 
-// Order 4: the cubic Lagrange weights (-1, 9, 9, -1)/16 on cells I-2 .. I+1
-// along each direction, applied direction i first, then j, then k, for the
-// three cyclic orders (i, j, k) = (x, y, z), (y, z, x), (z, x, y), all
-// twelve final terms accumulated in one running sum, divided by 3.
-AXB_D double c2v4(const double *__restrict__ f, long long I, const long long st[3]) {
-  const double wt[4] = {-1.0 / 16.0, 9.0 / 16.0, 9.0 / 16.0, -1.0 / 16.0};
-  double avg = 0.0;
-#pragma unroll 1
-  for (int i = 0; i < 3; ++i) {
-    const int j = (i == 0) ? 1 : ((i == 1) ? 2 : 0);
-    const int k = (i == 0) ? 2 : ((i == 1) ? 0 : 1);
-    double gj[4];
-#pragma unroll
-    for (int dk = 0; dk < 4; ++dk) {
-      double gi[4];
-#pragma unroll
-      for (int dj = 0; dj < 4; ++dj) {
-        double s = 0.0;
-        const long long base = I + st[j] * (dj - 2) + st[k] * (dk - 2);
-#pragma unroll
-        for (int di = 0; di < 4; ++di)
-          s += wt[di] * __ldg(f + base + st[i] * (di - 2));
-        gi[dj] = s;
-      }
-      double s = 0.0;
-#pragma unroll
-      for (int dj = 0; dj < 4; ++dj)
-        s += wt[dj] * gi[dj];
-      gj[dk] = s;
-    }
-#pragma unroll
-    for (int dk = 0; dk < 4; ++dk)
-      avg += wt[dk] * gj[dk];
-  }
-  return avg / 3.0;
-}
-
-template <int ORDER>
-AXB_D double c2v(const double *__restrict__ f, long long I, const long long st[3]) {
-  if constexpr (ORDER == 2)
-    return c2v2(f, I, st[1], st[2]);
-  else
-    return c2v4(f, I, st);
-}
-
-// Interior vertices [ng, ng + n] per axis; x along the block's threads.
-template <int ORDER, bool ZVEC>
-__global__ void __launch_bounds__(128) k_tmunu(const TmunuArgs a) {
-  const BoxDev &b = a.b;
-  const int i = b.ng + blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = b.ng + blockIdx.y;
-  const int k = b.ng + blockIdx.z;
-  if (i > b.ng + b.n[0])
-    return;
-  const long long I = b.at(i, j, k);
-  const long long st[3] = {1, b.sy, b.sz};
-
-  const double rho_avg = c2v<ORDER>(a.rho, I, st);
-  const double eps_avg = c2v<ORDER>(a.eps, I, st);
-  const double press_avg = c2v<ORDER>(a.press, I, st);
-  double Bup[3];
-  for (int d = 0; d < 3; ++d)
-    Bup[d] = c2v<ORDER>(a.B[d], I, st);
-
+// T_{mu nu} of the fluid interpolated to vertex I (rho, eps, press, B^i and
+// v^i or z^i), added to the arrays (tmunu.cxx:76-178).
+template <bool ZVEC>
+AXB_D void tmunu_point(const TmunuArgs &a, long long I, double rho_avg, double eps_avg,
+                       double press_avg, const double (&Bup)[3], const double (&vz)[3]) {
   const sym3 g{__ldg(a.g[0] + I), __ldg(a.g[1] + I), __ldg(a.g[2] + I),
                __ldg(a.g[3] + I), __ldg(a.g[4] + I), __ldg(a.g[5] + I)};
   const double alp = __ldg(a.alp + I);
@@ -124,17 +65,15 @@ __global__ void __launch_bounds__(128) k_tmunu(const TmunuArgs a) {
   double vup[3], vlow[3], w;
   if constexpr (!ZVEC) {
     for (int d = 0; d < 3; ++d)
-      vup[d] = c2v<ORDER>(a.v[d], I, st);
+      vup[d] = vz[d];
     lower3(g, vup, vlow);
     w = 1.0 / sqrt(1.0 - dot3(vup, vlow));
   } else {
-    double zup[3], zlow[3];
-    for (int d = 0; d < 3; ++d)
-      zup[d] = c2v<ORDER>(a.v[d], I, st);
-    lower3(g, zup, zlow);
-    w = sqrt(1.0 + dot3(zup, zlow));
+    double zlow[3];
+    lower3(g, vz, zlow);
+    w = sqrt(1.0 + dot3(vz, zlow));
     for (int d = 0; d < 3; ++d) {
-      vup[d] = zup[d] / w;
+      vup[d] = vz[d] / w;
       vlow[d] = zlow[d] / w;
     }
   }
@@ -174,10 +113,179 @@ __global__ void __launch_bounds__(128) k_tmunu(const TmunuArgs a) {
     a.eT[c][I] = a.eT[c][I] + t[c];
 }
 
-template <int ORDER, bool ZVEC>
-void launch_tmunu(const TmunuArgs &a, cudaStream_t s) {
-  const dim3 grid((a.b.n[0] + 1 + 127) / 128, a.b.n[1] + 1, a.b.n[2] + 1);
-  k_tmunu<ORDER, ZVEC><<<grid, 128, 0, s>>>(a);
+// Order 2: one thread per interior vertex [ng, ng + n]; x along the block's
+// threads, the 8 cells around a vertex from L1/L2.
+template <bool ZVEC> __global__ void __launch_bounds__(128) k_tmunu2(const TmunuArgs a) {
+  const BoxDev &b = a.b;
+  const int i = b.ng + blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = b.ng + blockIdx.y;
+  const int k = b.ng + blockIdx.z;
+  if (i > b.ng + b.n[0])
+    return;
+  const long long I = b.at(i, j, k);
+  double q[9];
+#pragma unroll
+  for (int v = 0; v < 9; ++v)
+    q[v] = c2v2(a.f[v], I, b.sy, b.sz);
+  const double B[3] = {q[3], q[4], q[5]}, vz[3] = {q[6], q[7], q[8]};
+  tmunu_point<ZVEC>(a, I, q[0], q[1], q[2], B, vz);
+}
+
+// Order 4: the cubic Lagrange weights (-1, 9, 9, -1)/16 on cells I-2 .. I+1
+// along each direction, applied direction i first, then j, then k, for the
+// three cyclic orders (i, j, k) = (x, y, z), (y, z, x), (z, x, y), all
+// twelve final terms accumulated in one running sum, divided by 3.
+//
+// A vertex alone needs 3 x 64 loads and 3 x 84 multiply-adds per field (one
+// thread per vertex ran 4.5 k FP64 operations and 1.7 k loads, bound by L1
+// and by instruction fetch: 2635 us for 129^3 vertices against 104 us of
+// HBM traffic; now 611 us, bound by the shared-memory and shuffle traffic of
+// 16 warps per SM).  The first- and second-direction sums of one vertex are those
+// of its neighbours, so a block forms each once: a tile of 29 x 13 x 3
+// vertices, 32 lanes along x (x sums by shuffles), 16 rows along y (y sums
+// through shared memory), 6 planes in z per thread (z sums in registers).
+// Every sum is the same terms in the same order as before, so the bits are
+// the same.  One field at a time through a rolled loop (the code of nine
+// unrolled fields does not fit the instruction cache), its results parked in
+// the thread's own shared-memory slots; the next field's loads are issued
+// ahead of this one's sums.
+constexpr int T4_X = 29, T4_Y = 13, T4_Z = 3; // vertices of a tile
+constexpr int T4_ROWS = T4_Y + 3, T4_P = T4_Z + 3;
+constexpr int T4_N = 32 * T4_ROWS; // threads
+constexpr int T4_SMEM = (2 * T4_P + T4_Z + 9 * T4_Z) * T4_N * int(sizeof(double));
+
+AXB_D double cubic(double a, double b, double c, double d) {
+  double s = -1.0 / 16.0 * a;
+  s += 9.0 / 16.0 * b;
+  s += 9.0 / 16.0 * c;
+  s += -1.0 / 16.0 * d;
+  return s;
+}
+// the cubic sum over lanes l-2 .. l+1 (lanes 2 .. 30 get theirs)
+AXB_D double cubic_x(double v) {
+  const double a = __shfl_up_sync(0xffffffffu, v, 2), b = __shfl_up_sync(0xffffffffu, v, 1),
+               d = __shfl_down_sync(0xffffffffu, v, 1);
+  return cubic(a, b, v, d);
+}
+// the cubic sum over rows r-2 .. r+1 of the plane at p (this thread's slot;
+// `v` is its own value); rows without all four neighbours get no sum
+AXB_D double cubic_y(const double *p, double v, bool ok) {
+  return ok ? cubic(p[-64], p[-32], v, p[32]) : 0.0;
+}
+
+template <bool ZVEC> __global__ void __launch_bounds__(T4_N, 1) k_tmunu4(const TmunuArgs a) {
+  extern __shared__ double sm[];
+  const BoxDev &b = a.b;
+  const int lane = threadIdx.x, row = threadIdx.y;
+  const int t = row * 32 + lane;
+  double *const s_f = sm + t;                  // the field's planes
+  double *const s_x = s_f + T4_P * T4_N;       // their x sums
+  double *const s_zx = s_x + T4_P * T4_N;      // x sums of the z sums
+  double *const s_res = s_zx + T4_Z * T4_N;    // results, field by field
+  const int i = b.ng + int(blockIdx.x) * T4_X + lane - 2;
+  const int j = b.ng + int(blockIdx.y) * T4_Y + row - 2;
+  const int k0 = b.ng + int(blockIdx.z) * T4_Z;
+  // cells past ng + n + 1 are needed by no vertex of the box
+  long long at[T4_P];
+#pragma unroll
+  for (int p = 0; p < T4_P; ++p)
+    at[p] = b.at(min(i, b.ng + b.n[0] + 1), min(j, b.ng + b.n[1] + 1),
+                 min(k0 - 2 + p, b.ng + b.n[2] + 1));
+  const bool row_ok = row >= 2 && row < T4_ROWS - 1;
+  double f[T4_P], fn[T4_P];
+#pragma unroll
+  for (int p = 0; p < T4_P; ++p)
+    fn[p] = __ldg(a.f[0] + at[p]);
+#pragma unroll 1
+  for (int v = 0; v < 9; ++v) {
+#pragma unroll
+    for (int p = 0; p < T4_P; ++p)
+      f[p] = fn[p];
+    if (v < 8) {
+      const double *nf = a.f[v + 1];
+#pragma unroll
+      for (int p = 0; p < T4_P; ++p)
+        fn[p] = __ldg(nf + at[p]);
+    }
+    double gx[T4_P], gzx[T4_Z];
+#pragma unroll
+    for (int p = 0; p < T4_P; ++p)
+      gx[p] = cubic_x(f[p]);
+#pragma unroll
+    for (int q = 0; q < T4_Z; ++q)
+      gzx[q] = cubic_x(cubic(f[q], f[q + 1], f[q + 2], f[q + 3]));
+    __syncthreads(); // the previous field's sums are read
+#pragma unroll
+    for (int p = 0; p < T4_P; ++p) {
+      s_f[p * T4_N] = f[p];
+      s_x[p * T4_N] = gx[p];
+    }
+#pragma unroll
+    for (int q = 0; q < T4_Z; ++q)
+      s_zx[q * T4_N] = gzx[q];
+    __syncthreads();
+    double avg[T4_Z], gy[T4_P];
+    // (x, y, z): the y sums of the x sums, summed over z
+    {
+      double gxy[T4_P];
+#pragma unroll
+      for (int p = 0; p < T4_P; ++p)
+        gxy[p] = cubic_y(s_x + p * T4_N, gx[p], row_ok);
+#pragma unroll
+      for (int q = 0; q < T4_Z; ++q)
+        avg[q] = cubic(gxy[q], gxy[q + 1], gxy[q + 2], gxy[q + 3]);
+    }
+    // (y, z, x): the z sums of the y sums, summed over x
+#pragma unroll
+    for (int p = 0; p < T4_P; ++p)
+      gy[p] = cubic_y(s_f + p * T4_N, f[p], row_ok);
+#pragma unroll
+    for (int q = 0; q < T4_Z; ++q) {
+      const double s = cubic(gy[q], gy[q + 1], gy[q + 2], gy[q + 3]);
+      const double sa = __shfl_up_sync(0xffffffffu, s, 2), sb = __shfl_up_sync(0xffffffffu, s, 1),
+                   sd = __shfl_down_sync(0xffffffffu, s, 1);
+      avg[q] += -1.0 / 16.0 * sa;
+      avg[q] += 9.0 / 16.0 * sb;
+      avg[q] += 9.0 / 16.0 * s;
+      avg[q] += -1.0 / 16.0 * sd;
+    }
+    // (z, x, y): the x sums of the z sums, summed over y
+    if (row_ok) {
+#pragma unroll
+      for (int q = 0; q < T4_Z; ++q) {
+        const double *p = s_zx + q * T4_N;
+        avg[q] += -1.0 / 16.0 * p[-64];
+        avg[q] += 9.0 / 16.0 * p[-32];
+        avg[q] += 9.0 / 16.0 * gzx[q];
+        avg[q] += -1.0 / 16.0 * p[32];
+        s_res[(v * T4_Z + q) * T4_N] = avg[q] / 3.0;
+      }
+    }
+  }
+  if (!row_ok || lane < 2 || lane > 30 || i > b.ng + b.n[0] || j > b.ng + b.n[1])
+    return;
+#pragma unroll 1
+  for (int q = 0; q < T4_Z; ++q) {
+    if (k0 + q > b.ng + b.n[2])
+      break;
+    auto res = [&](int v) { return s_res[(v * T4_Z + q) * T4_N]; };
+    const double B[3] = {res(3), res(4), res(5)}, vz[3] = {res(6), res(7), res(8)};
+    tmunu_point<ZVEC>(a, b.at(i, j, k0 + q), res(0), res(1), res(2), B, vz);
+  }
+}
+
+template <bool ZVEC> int launch_tmunu(int order, const TmunuArgs &a, cudaStream_t s) {
+  const int *n = a.b.n;
+  if (order == 2) {
+    k_tmunu2<ZVEC><<<dim3((n[0] + 1 + 127) / 128, n[1] + 1, n[2] + 1), 128, 0, s>>>(a);
+    return AXB_OK;
+  }
+  if (cudaFuncSetAttribute(k_tmunu4<ZVEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           T4_SMEM) != cudaSuccess)
+    return AXB_ERR_CUDA;
+  const dim3 grid((n[0] + T4_X) / T4_X, (n[1] + T4_Y) / T4_Y, (n[2] + T4_Z) / T4_Z);
+  k_tmunu4<ZVEC><<<grid, dim3(32, T4_ROWS), T4_SMEM, s>>>(a);
+  return AXB_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -287,15 +395,15 @@ AXB_API int axb_tmunu(axb_ctx *c, const axb_box *box, const axb_fields *f,
   for (const double *q : req)
     if (!q)
       return AXB_ERR_ARG;
-  a.rho = f->gf[AXB_GF_rho];
-  a.eps = f->gf[AXB_GF_eps];
-  a.press = f->gf[AXB_GF_press];
+  a.f[0] = f->gf[AXB_GF_rho];
+  a.f[1] = f->gf[AXB_GF_eps];
+  a.f[2] = f->gf[AXB_GF_press];
   a.alp = f->gf[AXB_GF_alp];
   for (int d = 0; d < 3; ++d) {
-    a.v[d] = f->gf[(zv ? AXB_GF_zvec_x : AXB_GF_velx) + d];
-    a.B[d] = f->gf[AXB_GF_Bvecx + d];
+    a.f[3 + d] = f->gf[AXB_GF_Bvecx + d];
+    a.f[6 + d] = f->gf[(zv ? AXB_GF_zvec_x : AXB_GF_velx) + d];
     a.beta[d] = f->gf[AXB_GF_betax + d];
-    if (!a.v[d] || !a.B[d] || !a.beta[d])
+    if (!a.f[3 + d] || !a.f[6 + d] || !a.beta[d])
       return AXB_ERR_ARG;
   }
   for (int q = 0; q < 6; ++q) {
@@ -310,11 +418,11 @@ AXB_API int axb_tmunu(axb_ctx *c, const axb_box *box, const axb_fields *f,
   }
   cudaStream_t s = (cudaStream_t)stream;
   axb_mark(c, AXB_R_TMUNU, s, true);
-  if (interp_order == 2)
-    zv ? launch_tmunu<2, true>(a, s) : launch_tmunu<2, false>(a, s);
-  else
-    zv ? launch_tmunu<4, true>(a, s) : launch_tmunu<4, false>(a, s);
+  const int rc = zv ? launch_tmunu<true>(interp_order, a, s)
+                    : launch_tmunu<false>(interp_order, a, s);
   axb_mark(c, AXB_R_TMUNU, s, false);
+  if (rc)
+    return rc;
   return cudaGetLastError() == cudaSuccess ? AXB_OK : AXB_ERR_CUDA;
 }
 
