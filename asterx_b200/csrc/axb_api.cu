@@ -447,6 +447,16 @@ AXB_API int axb_eos_create_tabulated3d(int nrho, int ntemp, int nye,
     emax = std::fmax(emax, v);
   }
   t.rgeps = Range{std::fmax(emin, 1e-15), emax};
+  // neighbouring temperature nodes further apart in ln eps than the bilinear
+  // interpolation's rounding (a few 1e-16 of the largest value)
+  double ymax = 0;
+  for (size_t q = 0; q < nodes; ++q)
+    ymax = std::fmax(ymax, std::fabs(hy[TAB_NV * q + TAB_EPS]));
+  t.monotone = 1;
+  for (size_t q = 0; q < nodes; ++q)
+    if ((q / nrho) % ntemp + 1 < size_t(ntemp) &&
+        !(hy[TAB_NV * (q + nrho) + TAB_EPS] - hy[TAB_NV * q + TAB_EPS] > 1e-12 * ymax))
+      t.monotone = 0;
   t.err = nullptr;
   if (cudaMemcpy(dptr, h, total * sizeof(double), cudaMemcpyHostToDevice) !=
       cudaSuccess) {

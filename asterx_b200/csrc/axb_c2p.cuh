@@ -587,28 +587,37 @@ template <class F>
 AXB_HD bool brent_step(BrentState &st, const F &f, double eps, int maxiters, double &lo,
                        double &hi) {
   double a = st.a, b = st.b, c = st.c, d = st.d, fa = st.fa, fb = st.fb, fc = st.fc;
-  if (st.iters >= maxiters || fabs(b - a) <= eps * fmin(fabs(a), fabs(b))) {
+  const double aa = fabs(a), ab = fabs(b);
+  if (st.iters >= maxiters || fabs(b - a) <= eps * (aa < ab ? aa : ab)) {
     lo = fmin(a, b);
     hi = fmax(a, b);
     return true;
   }
   ++st.iters;
-  double s;
-  if (fa != fc && fb != fc) {
-    // inverse quadratic interpolation over one common denominator
-    // (fa-fb)(fa-fc)(fb-fc) instead of three (last-ulp differences)
+  // inverse quadratic interpolation over one common denominator
+  // (fa-fb)(fa-fc)(fb-fc) instead of three (last-ulp differences), or the
+  // secant; the division of either in one place, so that lanes on both sides
+  // of the choice share it
+  const bool iqi = fa != fc && fb != fc;
+  double num, den;
+  if (iqi) {
     const double dab = fa - fb, dac = fa - fc, dbc = fb - fc;
-    s = (a * fb * fc * dbc - b * fa * fc * dac + c * fa * fb * dab) / (dab * dac * dbc);
+    num = a * fb * fc * dbc - b * fa * fc * dac + c * fa * fb * dab;
+    den = dab * dac * dbc;
   } else {
-    s = b - fb * (b - a) / (fb - fa);
+    num = fb * (b - a);
+    den = fb - fa;
   }
+  const double ratio = num / den;
+  double s = iqi ? ratio : b - ratio;
   const double delta = eps * fabs(b);
   const double q = (3 * a + b) / 4;
   const bool mflag = st.mflag;
-  const bool out_of_range = !((s > fmin(q, b)) && (s < fmax(q, b)));
-  if (out_of_range || (mflag && fabs(s - b) >= fabs(b - c) / 2) ||
-      (!mflag && fabs(s - b) >= fabs(c - d) / 2) || (mflag && fabs(b - c) < delta) ||
-      (!mflag && fabs(c - d) < delta)) {
+  // s strictly between q and b, in either order (false for a NaN)
+  const bool in_range = (s > q && s < b) || (s > b && s < q);
+  // the step before last (or the last) bounds this one
+  const double last = mflag ? fabs(b - c) : fabs(c - d);
+  if (!in_range || fabs(s - b) >= last / 2 || last < delta) {
     s = (a + b) / 2;
     st.mflag = true;
   } else {
@@ -680,122 +689,111 @@ struct PalQRST {
 // division, and P/rho comes from the EOS without a division (last-ulp
 // differences; the bracket search converges to the same tolerance).
 template <class EOS>
-AXB_HD double pal_froot(const EOS &eos, const C2PParams &cp, const Atmo &atmo,
-                        const PalQRST &k, double x, const Cons &cv) {
+AXB_HD double pal_froot(const EOS &eos, const C2PParams &cp, double atmo_eps,
+                        const PalQRST &k, double x, double dens, int &hint) {
   const double xs = x + k.s;
   const double ixxs = 1.0 / (x * xs); // 1/(x (x+s)); 1/x = (x+s)/(x (x+s))
   const double ix = xs * ixxs;
   double Wminus2 = 1.0 - (x * x * k.r + (2.0 * x + k.s) * k.t * k.t) * (ixxs * ixxs);
-  Wminus2 = fmin(fmax(Wminus2, 1e-10), 1);
+  // the clamps as selects (a NaN becomes 1e-10, as fmax makes it)
+  Wminus2 = Wminus2 > 1e-10 ? Wminus2 : 1e-10;
+  Wminus2 = Wminus2 < 1.0 ? Wminus2 : 1.0;
   const double W_loc = rsqrt(Wminus2);
   const double iW = Wminus2 * W_loc;
-  const double rho_loc = cv.dens * iW;
+  const double rho_loc = dens * iW;
   const double Ye_loc = k.ye;
   double eps_loc = W_loc - 1.0 + (1.0 - W_loc * W_loc) * x * iW +
                    W_loc * (k.q - k.s + 0.5 * k.t * k.t * (ix * ix) + 0.5 * k.s * Wminus2);
   if (cp.use_temp) {
-    eps_loc = fmax(eps_loc, atmo.eps);
+    eps_loc = fmax(eps_loc, atmo_eps);
     eps_loc = fmin(eps_loc, eos.rgeps.max);
   }
-  return (x - (1.0 + eps_loc + eos.press_over_rho(rho_loc, eps_loc, Ye_loc)) * W_loc);
+  return (x - (1.0 + eps_loc + eos.press_over_rho(rho_loc, eps_loc, Ye_loc, hint)) * W_loc);
 }
 
-// Palenzuela 1D (c2p_1DPalenzuela::solve, c2p_1DPalenzuela.hxx:306-556).
-// `xlo`/`xhi` > 0 narrow the initial bracket (learned initial guess); the
-// reference bracket is used when they are negative or do not bracket.
-// FAST: the common path only -- every failure, and a bracket that did not
-// converge (which needs the conservative-variable check), returns REP_DEFER
-// before anything else, so the caller can hand the cell to the full cascade.
-template <class EOS, bool FAST = false>
-AXB_HD void palenzuela_solve(const EOS &eos, const C2PParams &cp, const Atmo &atmo,
-                             Prim &pv, Cons &cv, const sym3 &glo, Report &rep,
-                             double xlo = -1.0, double xhi = -1.0) {
-  rep.iters = 0;
-  rep.adjust_cons = false;
-  rep.set_atmo = false;
-  rep.status = REP_SUCCESS;
+// What the Palenzuela scheme carries from its set-up to its solution: the
+// undensitised invariants, the initial bracket and the root function there.
+struct PalSetup {
+  double sqrt_detg, Bsq, BiSi;
+  PalQRST k;
+  double a, b, fa, fb;
+  int hint; // the tabulated EOS's temperature cell
+};
+
+// c2p_1DPalenzuela.hxx:306-401: checks, undensitised conserved variables,
+// invariants and the bracket.  Returns REP_SUCCESS or the failure's code
+// (the caller sets the cell's values to NaN).  `xlo`/`xhi` > 0 narrow the
+// initial bracket (learned initial guess); the reference bracket is used when
+// they are negative or do not bracket.
+template <class EOS>
+AXB_HD int pal_setup(const EOS &eos, const C2PParams &cp, const Atmo &atmo, Cons &cv,
+                     const sym3 &glo, sym3 &gup, double xlo, double xhi, PalSetup &o) {
   const double spatial_detg = det3(glo);
-  const double sqrt_detg = sqrt(spatial_detg);
+  o.sqrt_detg = sqrt(spatial_detg);
   const bool minor1 = glo.xx > 0.0;
   const bool minor2 = glo.xx * glo.yy - glo.xy * glo.xy > 0.0;
   const bool minor3 = spatial_detg > 0.0;
-  if (!(minor1 && minor2 && minor3)) {
-    if constexpr (FAST) {
-      rep.status = REP_DEFER;
-      return;
-    }
-    rep.fail(REP_INVALID_DETG);
-    pv.set_nan();
-    cv.set_nan();
-    return;
-  }
-  const sym3 gup = inv3(glo, spatial_detg);
-  cv.unscale(sqrt_detg);
+  if (!(minor1 && minor2 && minor3))
+    return REP_INVALID_DETG;
+  gup = inv3(glo, spatial_detg);
+  cv.unscale(o.sqrt_detg);
   double mom_up[3];
   lower3(gup, cv.mom, mom_up);
   const double Ssq = cv.mom[0] * mom_up[0] + cv.mom[1] * mom_up[1] + cv.mom[2] * mom_up[2];
   double B_low[3];
   lower3(glo, cv.dBvec, B_low);
-  const double Bsq = dot3(B_low, cv.dBvec);
-  const double BiSi =
-      cv.dBvec[0] * cv.mom[0] + cv.dBvec[1] * cv.mom[1] + cv.dBvec[2] * cv.mom[2];
-  if (!isfinite(cv.dens) || !isfinite(Ssq) || !isfinite(Bsq) || !isfinite(BiSi) ||
-      !isfinite(cv.DYe) || !isfinite(cv.DEnt)) {
-    if constexpr (FAST) {
-      rep.status = REP_DEFER;
-      return;
-    }
-    rep.fail(REP_NANS_IN_CONS);
-    pv.set_nan();
-    cv.set_nan();
-    return;
-  }
-  if (Bsq > cp.Bsq_lim) {
-    if constexpr (FAST) {
-      rep.status = REP_DEFER;
-      return;
-    }
-    rep.fail(REP_B_LIMIT);
-    pv.set_nan();
-    cv.set_nan();
-    return;
-  }
+  o.Bsq = dot3(B_low, cv.dBvec);
+  o.BiSi = cv.dBvec[0] * cv.mom[0] + cv.dBvec[1] * cv.mom[1] + cv.dBvec[2] * cv.mom[2];
+  if (!isfinite(cv.dens) || !isfinite(Ssq) || !isfinite(o.Bsq) || !isfinite(o.BiSi) ||
+      !isfinite(cv.DYe) || !isfinite(cv.DEnt))
+    return REP_NANS_IN_CONS;
+  if (o.Bsq > cp.Bsq_lim)
+    return REP_B_LIMIT;
   // the invariants as products with 1/dens and dens^(-1/2) = rsqrt(dens)
   // instead of five divisions and a pow (last-ulp differences)
   const double idens = 1.0 / cv.dens;
-  PalQRST k;
+  PalQRST &k = o.k;
   k.q = cv.tau * idens;
   k.r = Ssq * (idens * idens);
-  k.s = Bsq * idens;
-  k.t = BiSi * (idens * rsqrt(cv.dens));
+  k.s = o.Bsq * idens;
+  k.t = o.BiSi * (idens * rsqrt(cv.dens));
   k.ye = cv.DYe * idens;
   const double qP = k.q;
   const double sP = k.s;
-  double a = fmax(1e-10, 1.0 + qP - sP);
-  double b = 2.0 + 2.0 * qP - sP;
-  auto fn = [&](double x) { return pal_froot(eos, cp, atmo, k, x, cv); };
-  bool narrowed = false;
-  double fa = 0.0, fb = 0.0;
+  o.a = fmax(1e-10, 1.0 + qP - sP);
+  o.b = 2.0 + 2.0 * qP - sP;
+  o.hint = -1;
+  auto fn = [&](double x) { return pal_froot(eos, cp, atmo.eps, k, x, cv.dens, o.hint); };
   if (xlo > 0.0 && xhi > xlo) {
     const double flo = fn(xlo), fhi = fn(xhi);
     if (flo * fhi < 0) {
-      a = xlo;
-      b = xhi;
-      fa = flo;
-      fb = fhi;
-      narrowed = true;
+      o.a = xlo;
+      o.b = xhi;
+      o.fa = flo;
+      o.fb = fhi;
+      return REP_SUCCESS;
     }
   }
-  if (!narrowed) {
-    fa = fn(a);
-    fb = fn(b);
-    if (fa * fb > 0) {
-      b = 3.0 + 3.0 * qP - 1.5 * sP;
-      fb = fn(b);
-    }
+  o.fa = fn(o.a);
+  o.fb = fn(o.b);
+  if (o.fa * o.fb > 0) {
+    o.b = 3.0 + 3.0 * qP - 1.5 * sP;
+    o.fb = fn(o.b);
   }
-  double r0, r1;
-  brent_bracket(fn, a, b, fa, fb, cp.minbits, cp.maxIter, rep.iters, r0, r1);
+  return REP_SUCCESS;
+}
+
+// c2p_1DPalenzuela.hxx:402-556: the primitives from the final bracket
+// (r0, r1), the checks, the floors, the conserved variables.
+// FAST: a bracket that did not converge (which needs the
+// conservative-variable check) and every failure return REP_DEFER before
+// anything else, so the caller can hand the cell to the full cascade.
+template <class EOS, bool FAST>
+AXB_HD void pal_finish(const EOS &eos, const C2PParams &cp, const Atmo &atmo, const PalSetup &o,
+                       double r0, double r1, Prim &pv, Cons &cv, const sym3 &glo,
+                       const sym3 &gup, Report &rep) {
+  const PalQRST &k = o.k;
+  const double sqrt_detg = o.sqrt_detg;
   const bool converged = !(fabs(r0 - r1) > cp.tolerance_0 * fmin(fabs(r0), fabs(r1)));
   if constexpr (FAST) {
     if (!converged) {
@@ -823,11 +821,9 @@ AXB_HD void palenzuela_solve(const EOS &eos, const C2PParams &cp, const Atmo &at
       pv.eps = fmin(pv.eps, eos.rgeps.max);
     }
     const double Z_Sol = x_sol * pv.rho * W_sol;
-    vel_from_Z(Z_Sol, W_sol, Bsq, BiSi, cp.use_zprim, pv, cv, gup, glo);
+    vel_from_Z(Z_Sol, W_sol, o.Bsq, o.BiSi, cp.use_zprim, pv, cv, gup, glo);
     pv.Ye = cv.DYe / cv.dens;
-    pv.press = eos.press_from_valid_rho_eps_ye(pv.rho, pv.eps, pv.Ye);
-    pv.temperature = eos.temp_from_valid_rho_eps_ye(pv.rho, pv.eps, pv.Ye);
-    pv.entropy = eos.kappa_from_valid_rho_eps_ye(pv.rho, pv.eps, pv.Ye);
+    eos.press_temp_entropy(pv.rho, pv.eps, pv.Ye, o.hint, pv.press, pv.temperature, pv.entropy);
     for (int i = 0; i < 3; ++i)
       pv.Bvec[i] = cv.dBvec[i];
     set_E(pv, gup);
@@ -885,6 +881,30 @@ AXB_HD void palenzuela_solve(const EOS &eos, const C2PParams &cp, const Atmo &at
     cons_from_prim(cv, pv, glo);
   else
     cv.scale(sqrt_detg);
+}
+
+// Palenzuela 1D (c2p_1DPalenzuela::solve, c2p_1DPalenzuela.hxx:306-556).
+template <class EOS>
+AXB_HD void palenzuela_solve(const EOS &eos, const C2PParams &cp, const Atmo &atmo,
+                             Prim &pv, Cons &cv, const sym3 &glo, Report &rep,
+                             double xlo = -1.0, double xhi = -1.0) {
+  rep.iters = 0;
+  rep.adjust_cons = false;
+  rep.set_atmo = false;
+  rep.status = REP_SUCCESS;
+  sym3 gup;
+  PalSetup o;
+  const int rc = pal_setup(eos, cp, atmo, cv, glo, gup, xlo, xhi, o);
+  if (rc != REP_SUCCESS) {
+    rep.fail(rc);
+    pv.set_nan();
+    cv.set_nan();
+    return;
+  }
+  auto fn = [&](double x) { return pal_froot(eos, cp, atmo.eps, o.k, x, cv.dens, o.hint); };
+  double r0, r1;
+  brent_bracket(fn, o.a, o.b, o.fa, o.fb, cp.minbits, cp.maxIter, rep.iters, r0, r1);
+  pal_finish<EOS, false>(eos, cp, atmo, o, r0, r1, pv, cv, glo, gup, rep);
 }
 
 // Root function of the entropy scheme (c2p_1DEntropy.hxx:262-303, Appendix

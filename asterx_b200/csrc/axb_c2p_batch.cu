@@ -12,22 +12,22 @@ __global__ void __launch_bounds__(128) k_bstag_batch(const C2PBoxArgs *args, con
 }
 template <class EOS>
 __global__ void __launch_bounds__(128, AXB_C2P_MINB)
-    k_c2p_box_batch(const C2PBoxArgs *args, const TileTable t, unsigned long long *ctr, const EOS eos) {
+    k_c2p_box_batch(const C2PBoxArgs *args, const TileTable t, unsigned long long *ctr, const __grid_constant__ EOS eos) {
   batch_loop(args, t, ctr, [&](const C2PBoxArgs &a, const uint3 bid) {
     c2p_box_body<EOS>(a, eos, bid);
   });
 }
 template <class EOS>
-__global__ void __launch_bounds__(128, AXB_C2P_FAST_MINB)
+__global__ void __launch_bounds__(128, c2p_fast_minb<EOS>)
     k_c2p_fast_batch(const C2PBoxArgs *args, const TileTable t, unsigned long long *ctr,
-                     const EOS eos, const C2PQueue q) {
+                     const __grid_constant__ EOS eos, const C2PQueue q) {
   batch_loop(args, t, ctr, [&](const C2PBoxArgs &a, const uint3 bid, int box) {
     c2p_fast_body<EOS>(a, eos, bid, box, q);
   });
 }
 template <class EOS>
 __global__ void __launch_bounds__(128, AXB_C2P_MINB)
-    k_c2p_deferred_batch(const C2PBoxArgs *args, const EOS eos, const C2PQueue q) {
+    k_c2p_deferred_batch(const C2PBoxArgs *args, const __grid_constant__ EOS eos, const C2PQueue q) {
   c2p_deferred_body([&](int box) -> const C2PBoxArgs & { return args[box]; }, eos, q);
 }
 template <class EOS>

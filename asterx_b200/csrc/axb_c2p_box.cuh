@@ -15,6 +15,7 @@
 #include <cstring>
 #include <limits>
 #include <new>
+#include <type_traits>
 
 #include "axb_batch.cuh"
 #include "axb_c2p.cuh"
@@ -168,224 +169,228 @@ AXB_D int after_both_failed(const EOS &eos, const C2PBoxArgs &a, const Atmo &atm
   return AXB_C2P_FAIL;
 }
 
-// One cell of AsterX_Con2Prim_typeEoS (con2prim.cxx:81-453), preceded by
-// AsterX_ComputedBFromdBstag (computeBfromA.cxx:67-85) for the same cell.
 #ifndef AXB_C2P_MINB
 #define AXB_C2P_MINB 4 // resident CTAs per SM the register budget must allow
 #endif
-#ifndef AXB_C2P_FAST_MINB
-#define AXB_C2P_FAST_MINB 7 // the fast pass: fewer live values, more warps
-#endif
+// The fast pass: fewer live values, more warps.  Resident CTAs per SM, measured
+// on 4.0M ideal-gas cells (7 / 8 / 9 / 10: 1.255 / 1.237 / 1.249 / 1.296 ms) and
+// 96^3 tabulated ones (7 / 8 / 9: 2.67 / 2.70 / 2.85 ms).
+template <class EOS> constexpr int c2p_fast_minb = EOS::kTabulated ? 7 : 8;
+
+// The inputs of one cell both passes share: AsterX_ComputedBFromdBstag
+// (computeBfromA.cxx:67-85), the atmosphere, the metric averaged from the
+// eight vertices (aster_interp.hxx:23-36) and the conserved variables.
+struct CellData {
+  long long I;
+  Atmo atmo;
+  double alp_avg, sqrt_detg;
+  sym3 glo;
+  Cons cv;
+  double Bup[3];
+};
+template <class EOS>
+AXB_D void c2p_gather(const C2PBoxArgs &a, const EOS &eos, int i, int j, int k, CellData &c) {
+  const BoxDev &b = a.b;
+  const long long I = c.I = b.at(i, j, k);
+  double dB[3];
+  dB[0] = 0.5 * (a.dBstag[0][I] + a.dBstag[0][I + 1]);
+  dB[1] = 0.5 * (a.dBstag[1][I] + a.dBstag[1][I + b.sy]);
+  dB[2] = 0.5 * (a.dBstag[2][I] + a.dBstag[2][I + b.sz]);
+  if (a.atmo_uniform) {
+    c.atmo = a.atmo_const;
+  } else {
+    const double x = b.xmin[0] + (i - b.ng + 0.5) * b.dx[0];
+    const double y = b.xmin[1] + (j - b.ng + 0.5) * b.dx[1];
+    const double z = b.xmin[2] + (k - b.ng + 0.5) * b.dx[2];
+    c.atmo = cell_atmosphere(a, eos, x, y, z);
+  }
+  auto v2c = [&](const double *f) {
+    double s = 0.0;
+    s += f[I];
+    s += f[I + 1];
+    s += f[I + b.sy];
+    s += f[I + 1 + b.sy];
+    s += f[I + b.sz];
+    s += f[I + 1 + b.sz];
+    s += f[I + b.sy + b.sz];
+    s += f[I + 1 + b.sy + b.sz];
+    return s / 8.0;
+  };
+  c.alp_avg = v2c(a.alp);
+  c.glo = sym3{v2c(a.g[0]), v2c(a.g[1]), v2c(a.g[2]), v2c(a.g[3]), v2c(a.g[4]), v2c(a.g[5])};
+  c.sqrt_detg = sqrt(det3(c.glo));
+  c.cv.dens = a.dens[I];
+  for (int q = 0; q < 3; ++q)
+    c.cv.mom[q] = a.mom[q][I];
+  c.cv.tau = a.tau[I];
+  c.cv.DYe = a.DYe[I];
+  c.cv.DEnt = a.DEnt[I];
+  for (int q = 0; q < 3; ++q)
+    c.cv.dBvec[q] = dB[q];
+  const double isg = 1.0 / c.sqrt_detg;
+  for (int q = 0; q < 3; ++q)
+    c.Bup[q] = c.cv.dBvec[q] * isg;
+}
+
+// A cell's results (con2prim.cxx:417-453).
+AXB_D void c2p_store(const C2PBoxArgs &a, long long I, int code, const Prim &pv, const Cons &cv) {
+  a.flag[I] = code;
+  a.rho[I] = pv.rho;
+  a.eps[I] = pv.eps;
+  a.Ye[I] = pv.Ye;
+  a.press[I] = pv.press;
+  a.temperature[I] = pv.temperature;
+  a.entropy[I] = pv.entropy;
+  for (int q = 0; q < 3; ++q) {
+    a.vel[q][I] = pv.vel[q];
+    a.Bvec[q][I] = pv.Bvec[q];
+  }
+  const double wlor = pv.w_lor;
+  const double hW2 = (pv.rho + pv.rho * pv.eps + pv.press) * wlor * wlor;
+  for (int q = 0; q < 3; ++q) {
+    if (a.zvec[q])
+      a.zvec[q][I] = wlor * pv.vel[q];
+    if (a.svec[q])
+      a.svec[q][I] = hW2 * pv.vel[q];
+  }
+  a.dens[I] = cv.dens;
+  for (int q = 0; q < 3; ++q)
+    a.mom[q][I] = cv.mom[q];
+  a.tau[I] = cv.tau;
+  a.DYe[I] = cv.DYe;
+  a.DEnt[I] = cv.DEnt;
+  for (int q = 0; q < 3; ++q)
+    if (a.dB[q])
+      a.dB[q][I] = cv.dBvec[q];
+  a.saved_rho[I] = pv.rho;
+  for (int q = 0; q < 3; ++q)
+    a.saved_vel[q][I] = pv.vel[q];
+  a.saved_eps[I] = pv.eps;
+  a.saved_Ye[I] = pv.Ye;
+}
+
+// The first solver's start from the learned guess (x, W) of a cell: the Noble
+// seeds Z = D x, v^2 = 1 - 1/W^2 and the Palenzuela bracket x (1 -+ bracket);
+// all -1 when the guess is unusable.
+struct GuessStart {
+  double z = -1.0, vsq = -1.0, xlo = -1.0, xhi = -1.0;
+};
+AXB_D GuessStart guess_start(const C2PBoxArgs &a, int i, int j, int k, const CellData &c) {
+  const BoxDev &b = a.b;
+  const long long ci = ((long long)(k - b.ng) * b.n[1] + (j - b.ng)) * b.n[0] + (i - b.ng);
+  const float2 gs = a.guess[ci];
+  const double x = gs.x, W = gs.y;
+  GuessStart g;
+  g.z = c.cv.dens / c.sqrt_detg * x; // Z = rho h W^2 = D (h W)
+  g.vsq = 1.0 - 1.0 / (W * W);
+  g.xlo = x * (1.0 - a.bracket);
+  g.xhi = x * (1.0 + a.bracket);
+  if (!(g.z > 0.0 && g.z < 1e300 && g.vsq >= 0.0 && g.vsq < 1.0))
+    g = GuessStart{};
+  return g;
+}
+
+// One cell of AsterX_Con2Prim_typeEoS (con2prim.cxx:81-453), the whole
+// cascade.
 //
-// MODE C2P_FULL runs the whole cascade.  MODE C2P_FAST (Palenzuela as the
-// first solver) runs the common path only and returns true, having written
-// nothing, for a cell that needs anything else -- the excision / BH-interior
-// treatment, a Palenzuela failure (and so the second solver), or a bracket
-// that did not converge (and so the conservative-variable check); such a
-// cell is then recovered by the full cascade in a second launch, from the
-// same unmodified inputs, so every cell gets exactly the full cascade's
-// result.  The rare paths' code stays out of the fast kernel and no warp of
-// it waits on them.
-//
-// GUESS (with a.guess): the first solver starts from the learned guess --
-// the Noble seeds Z = D x, v^2 = 1 - 1/W^2, or the Palenzuela bracket
-// x (1 -+ bracket).  A guessed first attempt that fails returns C2P_RETRY
-// having written nothing; the caller then runs the cell again without the
-// guess (the plain seeds, as c2p_2DNoble.hxx:374-393 and
-// c2p_1DPalenzuela.hxx:395-401 set them, and the plain cascade).
-enum { C2P_FULL = 0, C2P_FAST = 1 };
-enum { C2P_DONE = 0, C2P_DEFERRED = 1, C2P_RETRY = 2 };
-template <class EOS, int MODE, bool GUESS = false>
+// GUESS (with a.guess): the first solver starts from the learned guess.  A
+// guessed first attempt that fails returns C2P_RETRY having written nothing;
+// the caller then runs the cell again without the guess (the plain seeds, as
+// c2p_2DNoble.hxx:374-393 and c2p_1DPalenzuela.hxx:395-401 set them, and the
+// plain cascade).
+enum { C2P_DONE = 0, C2P_RETRY = 1 };
+template <class EOS, bool GUESS = false>
 AXB_D int c2p_cell(const C2PBoxArgs &a, const EOS &eos, const int i, const int j,
                    const int k, int &iters_first, bool &failed, bool use_guess = false) {
-  constexpr bool FASTLIKE = MODE == C2P_FAST;
-  const BoxDev &b = a.b;
-  {
-    const long long I = b.at(i, j, k);
-    double dB[3];
-    dB[0] = 0.5 * (a.dBstag[0][I] + a.dBstag[0][I + 1]);
-    dB[1] = 0.5 * (a.dBstag[1][I] + a.dBstag[1][I + b.sy]);
-    dB[2] = 0.5 * (a.dBstag[2][I] + a.dBstag[2][I + b.sz]);
-    Atmo atmo;
-    if (a.atmo_uniform) {
-      atmo = a.atmo_const;
-    } else {
-      const double x = b.xmin[0] + (i - b.ng + 0.5) * b.dx[0];
-      const double y = b.xmin[1] + (j - b.ng + 0.5) * b.dx[1];
-      const double z = b.xmin[2] + (k - b.ng + 0.5) * b.dx[2];
-      atmo = cell_atmosphere(a, eos, x, y, z);
-    }
-    // vertex-to-cell metric (aster_interp.hxx:23-36)
-    auto v2c = [&](const double *f) {
-      double s = 0.0;
-      s += f[I];
-      s += f[I + 1];
-      s += f[I + b.sy];
-      s += f[I + 1 + b.sy];
-      s += f[I + b.sz];
-      s += f[I + 1 + b.sz];
-      s += f[I + b.sy + b.sz];
-      s += f[I + 1 + b.sy + b.sz];
-      return s / 8.0;
-    };
-    const double alp_avg = v2c(a.alp);
-    const sym3 glo{v2c(a.g[0]), v2c(a.g[1]), v2c(a.g[2]),
-                   v2c(a.g[3]), v2c(a.g[4]), v2c(a.g[5])};
-    double mask_local = 1.0;
-    const double spatial_detg = det3(glo);
-    const double sqrt_detg = sqrt(spatial_detg);
-    double v_up[3] = {a.saved_vel[0][I], a.saved_vel[1][I], a.saved_vel[2][I]};
-    double v_low[3];
-    lower3(glo, v_up, v_low);
-    double zsq;
-    const double vsq = dot3(v_low, v_up);
-    if (vsq >= 1.0) {
-      const double wlim = sqrt(1.0 + a.cp.vw_lim * a.cp.vw_lim);
-      const double vlim = a.cp.vw_lim / wlim;
-      for (int q = 0; q < 3; ++q) {
-        v_up[q] *= vlim / sqrt(vsq);
-        v_low[q] *= vlim / sqrt(vsq);
-      }
-      zsq = a.cp.vw_lim * a.cp.vw_lim;
-    } else {
-      zsq = vsq / (1.0 - vsq);
-    }
-    double wlor = sqrt(1.0 + zsq);
-    Cons cv;
-    cv.dens = a.dens[I];
-    for (int q = 0; q < 3; ++q)
-      cv.mom[q] = a.mom[q][I];
-    cv.tau = a.tau[I];
-    cv.DYe = a.DYe[I];
-    cv.DEnt = a.DEnt[I];
-    for (int q = 0; q < 3; ++q)
-      cv.dBvec[q] = dB[q];
-    const double isg = 1.0 / sqrt_detg;
-    const double Bup[3] = {cv.dBvec[0] * isg, cv.dBvec[1] * isg, cv.dBvec[2] * isg};
-    Prim pv;
-    pv.set_nan();
-    Prim seeds;
-    seeds.rho = a.saved_rho[I];
-    seeds.eps = a.saved_eps[I];
-    seeds.Ye = a.saved_Ye[I];
-    {
-      double e = seeds.eps; // the reference clamps a copy, not the seed
-      seeds.press = eos.press_from_valid_rho_eps_ye(seeds.rho, e, seeds.Ye);
-    }
-    seeds.temperature = a.temperature[I];
-    seeds.entropy = 0.0; // only read by the excision path, filled there
+  CellData c;
+  c2p_gather(a, eos, i, j, k, c);
+  const long long I = c.I;
+  const Atmo &atmo = c.atmo;
+  const sym3 &glo = c.glo;
+  Cons &cv = c.cv;
+  double mask_local = 1.0;
+  double v_up[3] = {a.saved_vel[0][I], a.saved_vel[1][I], a.saved_vel[2][I]};
+  double v_low[3];
+  lower3(glo, v_up, v_low);
+  double zsq;
+  const double vsq = dot3(v_low, v_up);
+  if (vsq >= 1.0) {
+    const double wlim = sqrt(1.0 + a.cp.vw_lim * a.cp.vw_lim);
+    const double vlim = a.cp.vw_lim / wlim;
     for (int q = 0; q < 3; ++q) {
-      seeds.vel[q] = v_up[q];
-      seeds.Bvec[q] = Bup[q];
-      seeds.E[q] = 0.0;
+      v_up[q] *= vlim / sqrt(vsq);
+      v_low[q] *= vlim / sqrt(vsq);
     }
-    seeds.w_lor = wlor;
-    bool flag_local = true;
-    int code = AXB_C2P_INIT;
-    bool call_c2p = true;
-    if (cv.dens <= sqrt_detg * atmo.rho_cut) {
-      for (int q = 0; q < 3; ++q)
-        pv.Bvec[q] = Bup[q];
-      atmo.set(pv, cv, glo);
-      atmo.set(seeds);
-      code = AXB_C2P_ATMO;
-      call_c2p = false;
-    }
-    if (alp_avg < a.cp.alp_thresh)
-      mask_local = 0.0;
-    if constexpr (FASTLIKE) {
-      if (mask_local != 1.0)
-        return C2P_DEFERRED;
-    }
-    if (MODE == C2P_FULL && a.excise && mask_local != 1.0) {
-      seeds.entropy = eos.kappa_from_valid_rho_eps_ye(seeds.rho, seeds.eps, seeds.Ye);
-      bh_interior<false>(eos, a.cp, atmo, seeds, cv, glo);
-      pv = seeds;
-      call_c2p = false;
-    }
-    double zguess = -1.0, vsqguess = -1.0, xlo = -1.0, xhi = -1.0;
-    if constexpr (GUESS) {
-      if (use_guess && call_c2p) {
-        const long long ci =
-            ((long long)(k - b.ng) * b.n[1] + (j - b.ng)) * b.n[0] + (i - b.ng);
-        const float2 gs = a.guess[ci];
-        const double x = gs.x, W = gs.y;
-        zguess = cv.dens / sqrt_detg * x; // Z = rho h W^2 = D (h W)
-        vsqguess = 1.0 - 1.0 / (W * W);
-        xlo = x * (1.0 - a.bracket);
-        xhi = x * (1.0 + a.bracket);
-        if (!(zguess > 0.0 && zguess < 1e300 && vsqguess >= 0.0 && vsqguess < 1.0))
-          zguess = vsqguess = xlo = xhi = -1.0;
-      }
-    }
-    cons_floors(cv, glo);
-    if constexpr (FASTLIKE) {
-      if (call_c2p) {
-        Report r1;
-        code = AXB_C2P_PRIME;
-        palenzuela_solve<EOS, true>(eos, a.cp, atmo, pv, cv, glo, r1, xlo, xhi);
-        if (r1.failed())
-          return C2P_DEFERRED; // REP_DEFER: every failure goes to the full cascade
-        iters_first = r1.iters;
-      }
-    } else if (call_c2p) {
-      Report r1, r2;
-      code = AXB_C2P_PRIME;
-      if (GUESS && zguess >= 0.0) {
-        run_solver_guess(a.c2p_prime, eos, a, atmo, pv, seeds, cv, glo, r1, zguess, vsqguess,
-                         xlo, xhi);
-        if (r1.failed()) {
-          iters_first = r1.iters;
-          return C2P_RETRY;
-        }
-      } else {
-        run_solver(a.c2p_prime, eos, a, atmo, pv, seeds, cv, glo, r1);
-      }
-      iters_first = r1.iters;
-      if (r1.failed()) {
-        code = AXB_C2P_SECOND;
-        run_solver(a.c2p_second, eos, a, atmo, pv, seeds, cv, glo, r2);
-      }
-      if (r1.failed() && r2.failed())
-        code = after_both_failed(eos, a, atmo, mask_local, sqrt_detg, Bup, pv, seeds, cv, glo,
-                                 flag_local, failed);
-      if ((mask_local != 1.0) && flag_local)
-        bh_interior<true>(eos, a.cp, atmo, pv, cv, glo);
-    }
-    a.flag[I] = code;
-    a.rho[I] = pv.rho;
-    a.eps[I] = pv.eps;
-    a.Ye[I] = pv.Ye;
-    a.press[I] = pv.press;
-    a.temperature[I] = pv.temperature;
-    a.entropy[I] = pv.entropy;
-    for (int q = 0; q < 3; ++q) {
-      a.vel[q][I] = pv.vel[q];
-      a.Bvec[q][I] = pv.Bvec[q];
-    }
-    wlor = pv.w_lor;
-    const double hW2 = (pv.rho + pv.rho * pv.eps + pv.press) * wlor * wlor;
-    for (int q = 0; q < 3; ++q) {
-      if (a.zvec[q])
-        a.zvec[q][I] = wlor * pv.vel[q];
-      if (a.svec[q])
-        a.svec[q][I] = hW2 * pv.vel[q];
-    }
-    a.dens[I] = cv.dens;
-    for (int q = 0; q < 3; ++q)
-      a.mom[q][I] = cv.mom[q];
-    a.tau[I] = cv.tau;
-    a.DYe[I] = cv.DYe;
-    a.DEnt[I] = cv.DEnt;
-    for (int q = 0; q < 3; ++q)
-      if (a.dB[q])
-        a.dB[q][I] = cv.dBvec[q];
-    a.saved_rho[I] = pv.rho;
-    for (int q = 0; q < 3; ++q)
-      a.saved_vel[q][I] = pv.vel[q];
-    a.saved_eps[I] = pv.eps;
-    a.saved_Ye[I] = pv.Ye;
+    zsq = a.cp.vw_lim * a.cp.vw_lim;
+  } else {
+    zsq = vsq / (1.0 - vsq);
   }
+  Prim pv;
+  pv.set_nan();
+  Prim seeds;
+  seeds.rho = a.saved_rho[I];
+  seeds.eps = a.saved_eps[I];
+  seeds.Ye = a.saved_Ye[I];
+  {
+    double e = seeds.eps; // the reference clamps a copy, not the seed
+    seeds.press = eos.press_from_valid_rho_eps_ye(seeds.rho, e, seeds.Ye);
+  }
+  seeds.temperature = a.temperature[I];
+  seeds.entropy = 0.0; // only read by the excision path, filled there
+  for (int q = 0; q < 3; ++q) {
+    seeds.vel[q] = v_up[q];
+    seeds.Bvec[q] = c.Bup[q];
+    seeds.E[q] = 0.0;
+  }
+  seeds.w_lor = sqrt(1.0 + zsq);
+  bool flag_local = true;
+  int code = AXB_C2P_INIT;
+  bool call_c2p = true;
+  if (cv.dens <= c.sqrt_detg * atmo.rho_cut) {
+    for (int q = 0; q < 3; ++q)
+      pv.Bvec[q] = c.Bup[q];
+    atmo.set(pv, cv, glo);
+    atmo.set(seeds);
+    code = AXB_C2P_ATMO;
+    call_c2p = false;
+  }
+  if (c.alp_avg < a.cp.alp_thresh)
+    mask_local = 0.0;
+  if (a.excise && mask_local != 1.0) {
+    seeds.entropy = eos.kappa_from_valid_rho_eps_ye(seeds.rho, seeds.eps, seeds.Ye);
+    bh_interior<false>(eos, a.cp, atmo, seeds, cv, glo);
+    pv = seeds;
+    call_c2p = false;
+  }
+  GuessStart g;
+  if (GUESS && use_guess && call_c2p)
+    g = guess_start(a, i, j, k, c);
+  cons_floors(cv, glo);
+  if (call_c2p) {
+    Report r1, r2;
+    code = AXB_C2P_PRIME;
+    if (GUESS && g.z >= 0.0) {
+      run_solver_guess(a.c2p_prime, eos, a, atmo, pv, seeds, cv, glo, r1, g.z, g.vsq, g.xlo,
+                       g.xhi);
+      if (r1.failed()) {
+        iters_first = r1.iters;
+        return C2P_RETRY;
+      }
+    } else {
+      run_solver(a.c2p_prime, eos, a, atmo, pv, seeds, cv, glo, r1);
+    }
+    iters_first = r1.iters;
+    if (r1.failed()) {
+      code = AXB_C2P_SECOND;
+      run_solver(a.c2p_second, eos, a, atmo, pv, seeds, cv, glo, r2);
+    }
+    if (r1.failed() && r2.failed())
+      code = after_both_failed(eos, a, atmo, mask_local, c.sqrt_detg, c.Bup, pv, seeds, cv, glo,
+                               flag_local, failed);
+    if ((mask_local != 1.0) && flag_local)
+      bh_interior<true>(eos, a.cp, atmo, pv, cv, glo);
+  }
+  c2p_store(a, I, code, pv, cv);
   return C2P_DONE;
 }
 
@@ -426,7 +431,7 @@ AXB_D void c2p_cell_full(const C2PBoxArgs &a, const EOS &eos, int i, int j, int 
     int it0 = 0;
     for (int attempt = 0; attempt < 2; ++attempt) {
       const int rc =
-          c2p_cell<EOS, C2P_FULL, true>(a, eos, i, j, k, iters_first, failed, attempt == 0);
+          c2p_cell<EOS, true>(a, eos, i, j, k, iters_first, failed, attempt == 0);
       if (rc != C2P_RETRY) {
         if (attempt == 1 && iters_first >= 0)
           iters_first += it0;
@@ -435,7 +440,7 @@ AXB_D void c2p_cell_full(const C2PBoxArgs &a, const EOS &eos, int i, int j, int 
       it0 = iters_first;
     }
   } else {
-    c2p_cell<EOS, C2P_FULL>(a, eos, i, j, k, iters_first, failed);
+    c2p_cell<EOS>(a, eos, i, j, k, iters_first, failed);
   }
 }
 
@@ -454,7 +459,7 @@ AXB_D void c2p_box_body(const C2PBoxArgs &a, const EOS &eos, const uint3 bid) {
 }
 template <class EOS, bool GUESS = false>
 __global__ void __launch_bounds__(128, AXB_C2P_MINB)
-    k_c2p_box(const C2PBoxArgs a, const EOS eos) {
+    k_c2p_box(const C2PBoxArgs a, const __grid_constant__ EOS eos) {
   c2p_box_body<EOS, GUESS>(a, eos, blockIdx);
 }
 
@@ -485,24 +490,190 @@ AXB_D void queue_deferred(const C2PQueue &q, bool defer, int i, int j, int k, in
   }
 }
 
-// Fast pass over one tile: the common path, deferred cells appended to the
-// queue (warp-aggregated).
+// The root searches of a block's cells, drawn by its threads (tabulated EOS).
+//
+// Brent's method takes 4 to 40 steps (11 on average), so one cell per thread
+// leaves a warp running for its slowest cell (10.8 of 32 lanes at work).  Here
+// every cell's search is a record in shared memory (the invariants of its
+// root function and Brent's state).  All threads first run C2P_ROUND0 steps of
+// their own cells; then the unfinished searches are listed, the block's first
+// threads take them, run C2P_ROUND steps and put them back, until none is
+// left: the warps beyond the list wait at the barrier.  A search's steps are
+// the same whichever thread runs them.  A table's step (an inversion and
+// three logarithms or exponentials) is long enough to pay for it: 96^3 cells
+// 9.2 -> 2.7 ms together with the queries as function calls from a temperature
+// cell kept between steps (6 / 10 first and 6 further steps: the same).  An
+// ideal gas's step is not: 4.0M cells 1.24 ms one cell per thread, 1.46 ms
+// through the pool even without a second round (its records and barriers),
+// 1.51 ms with rounds.
+constexpr int C2P_ROUND0 = 8, C2P_ROUND = 4;
+constexpr int C2P_T = 128; // threads of a block
+template <class EOS> struct BrentPool {
+  enum { Q, R, S, T, AEPS, YE, DENS, A, B, C, D, FA, FB, FC, N };
+  double v[N][C2P_T];
+  int steps[C2P_T]; // steps taken, and Brent's flag in bit 0
+  int hint[C2P_T];
+  unsigned char list[C2P_T];
+  int count[C2P_T / 32];
+
+  AXB_D void put(int p, const BrentState &st) {
+    v[A][p] = st.a;
+    v[B][p] = st.b;
+    v[C][p] = st.c;
+    v[D][p] = st.d;
+    v[FA][p] = st.fa;
+    v[FB][p] = st.fb;
+    v[FC][p] = st.fc;
+    steps[p] = 2 * st.iters + (st.mflag ? 1 : 0);
+  }
+  // the cell's record; false when its bracket is final already
+  AXB_D bool init(int p, const PalSetup &o, double dens, double atmo_eps) {
+    BrentState st;
+    double lo, hi;
+    if (brent_init(st, o.a, o.b, o.fa, o.fb, lo, hi)) {
+      v[A][p] = lo;
+      v[B][p] = hi;
+      steps[p] = 0;
+      return false;
+    }
+    put(p, st);
+    v[Q][p] = o.k.q;
+    v[R][p] = o.k.r;
+    v[S][p] = o.k.s;
+    v[T][p] = o.k.t;
+    v[AEPS][p] = atmo_eps;
+    v[YE][p] = o.k.ye;
+    v[DENS][p] = dens;
+    hint[p] = o.hint;
+    return true;
+  }
+  // up to `nsteps` steps of record p; true when its bracket (A, B) is final
+  AXB_D bool advance(int p, int nsteps, const EOS &eos, const C2PParams &cp) {
+    BrentState st{v[A][p], v[B][p],  v[C][p],       v[D][p],            v[FA][p],
+                  v[FB][p], v[FC][p], steps[p] >> 1, (steps[p] & 1) != 0};
+    const PalQRST k{v[Q][p], v[R][p], v[S][p], v[T][p], v[YE][p]};
+    const double dens = v[DENS][p], aeps = v[AEPS][p];
+    int h = hint[p];
+    auto fn = [&](double x) { return pal_froot(eos, cp, aeps, k, x, dens, h); };
+    double lo, hi;
+    bool fin = false;
+    for (int q = 0; q < nsteps && !fin; ++q)
+      fin = brent_step(st, fn, cp.tolerance_0, cp.maxIter, lo, hi);
+    hint[p] = h;
+    if (fin) {
+      v[A][p] = lo;
+      v[B][p] = hi;
+      steps[p] = 2 * st.iters;
+    } else {
+      put(p, st);
+    }
+    return fin;
+  }
+  // every thread of the block calls; `live`: record threadIdx.x is open
+  AXB_D void run(bool live, const EOS &eos, const C2PParams &cp) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    int p = live ? t : -1;
+    __syncthreads(); // the last tile's counts are read
+    for (int n = C2P_ROUND0;; n = C2P_ROUND) {
+      const bool open = p >= 0 && !advance(p, n, eos, cp);
+      const unsigned m = __ballot_sync(0xffffffffu, open);
+      if (lane == 0)
+        count[warp] = __popc(m);
+      __syncthreads();
+      int before = 0, total = 0;
+#pragma unroll
+      for (int w = 0; w < C2P_T / 32; ++w) {
+        before += w < warp ? count[w] : 0;
+        total += count[w];
+      }
+      if (total == 0) // block-uniform
+        break;
+      if (open)
+        list[before + __popc(m & ((1u << lane) - 1u))] = (unsigned char)p;
+      __syncthreads();
+      p = t < total ? list[t] : -1;
+    }
+  }
+};
+
+// Fast pass over one tile (Palenzuela as the first solver): the common path
+// only.  A cell that needs anything else -- the excision / BH-interior
+// treatment, a Palenzuela failure (and so the second solver), or a bracket
+// that did not converge (and so the conservative-variable check) -- is queued
+// (warp-aggregated) with nothing written, and recovered by the full cascade in
+// a second launch from the same inputs, so every cell gets exactly the full
+// cascade's result.  The rare paths' code stays out of this kernel and no
+// warp of it waits on them.
 template <class EOS, bool GUESS = false>
 AXB_D void c2p_fast_body(const C2PBoxArgs &a, const EOS &eos, const uint3 bid, int box,
                          const C2PQueue &q) {
   __shared__ unsigned int s_hist[64];
+  constexpr bool POOL = EOS::kTabulated;
+  __shared__ std::conditional_t<POOL, BrentPool<EOS>, char> pool;
   c2p_hist_init(a, s_hist);
   int i, j;
   const int k = a.b.ng + bid.z;
   const bool in_range = a.b.row_ij(a.b.ng, a.b.n[0], a.b.ng, a.b.n[1], bid, i, j);
   int iters_first = -1;
-  bool failed = false;
-  bool defer = false;
-  if (in_range)
-    defer = c2p_cell<EOS, C2P_FAST, GUESS>(a, eos, i, j, k, iters_first, failed, GUESS) ==
-            C2P_DEFERRED;
+  bool defer = false, solve = false;
+  [[maybe_unused]] bool live = false;
+  CellData c;
+  PalSetup o;
+  sym3 gup;
+  if (in_range) {
+    c2p_gather(a, eos, i, j, k, c);
+    if (c.alp_avg < a.cp.alp_thresh) {
+      defer = true;
+    } else if (c.cv.dens <= c.sqrt_detg * c.atmo.rho_cut) {
+      Prim pv;
+      for (int d = 0; d < 3; ++d)
+        pv.Bvec[d] = c.Bup[d];
+      c.atmo.set(pv, c.cv, c.glo);
+      cons_floors(c.cv, c.glo);
+      c2p_store(a, c.I, AXB_C2P_ATMO, pv, c.cv);
+    } else {
+      GuessStart g;
+      if constexpr (GUESS)
+        g = guess_start(a, i, j, k, c);
+      cons_floors(c.cv, c.glo);
+      solve = pal_setup(eos, a.cp, c.atmo, c.cv, c.glo, gup, g.xlo, g.xhi, o) == REP_SUCCESS;
+      defer = !solve;
+      if constexpr (POOL)
+        live = solve && pool.init(threadIdx.x, o, c.cv.dens, c.atmo.eps);
+    }
+  }
+  if constexpr (POOL)
+    pool.run(live, eos, a.cp);
+  if (solve) {
+    Report rep;
+    rep.iters = 0;
+    rep.adjust_cons = false;
+    rep.set_atmo = false;
+    rep.status = REP_SUCCESS;
+    double r0, r1;
+    if constexpr (POOL) {
+      const int t = threadIdx.x;
+      o.hint = live ? pool.hint[t] : o.hint;
+      r0 = pool.v[pool.A][t];
+      r1 = pool.v[pool.B][t];
+      rep.iters = pool.steps[t] >> 1;
+    } else {
+      auto fn = [&](double x) {
+        return pal_froot(eos, a.cp, c.atmo.eps, o.k, x, c.cv.dens, o.hint);
+      };
+      brent_bracket(fn, o.a, o.b, o.fa, o.fb, a.cp.minbits, a.cp.maxIter, rep.iters, r0, r1);
+    }
+    Prim pv;
+    pal_finish<EOS, true>(eos, a.cp, c.atmo, o, r0, r1, pv, c.cv, c.glo, gup, rep);
+    if (rep.failed()) {
+      defer = true; // every failure goes to the full cascade
+    } else {
+      iters_first = rep.iters;
+      c2p_store(a, c.I, AXB_C2P_PRIME, pv, c.cv);
+    }
+  }
   queue_deferred(q, defer, i, j, k, box);
-  c2p_epilogue(a, s_hist, iters_first, failed);
+  c2p_epilogue(a, s_hist, iters_first, false);
 }
 
 // The full cascade over the queued cells; `args_of(box)` gives the box's
@@ -548,14 +719,14 @@ AXB_D void c2p_deferred_body(const ArgsOf &args_of, const EOS &eos, const C2PQue
 }
 
 template <class EOS, bool GUESS = false>
-__global__ void __launch_bounds__(128, AXB_C2P_FAST_MINB)
-    k_c2p_fast(const C2PBoxArgs a, const EOS eos, const C2PQueue q) {
+__global__ void __launch_bounds__(128, c2p_fast_minb<EOS>)
+    k_c2p_fast(const C2PBoxArgs a, const __grid_constant__ EOS eos, const C2PQueue q) {
   c2p_fast_body<EOS, GUESS>(a, eos, blockIdx, 0, q);
 }
 
 template <class EOS, bool GUESS = false>
 __global__ void __launch_bounds__(128, AXB_C2P_MINB)
-    k_c2p_deferred(const C2PBoxArgs a, const EOS eos, const C2PQueue q) {
+    k_c2p_deferred(const C2PBoxArgs a, const __grid_constant__ EOS eos, const C2PQueue q) {
   auto args_of = [&](int) -> const C2PBoxArgs & { return a; };
   c2p_deferred_body<EOS, decltype(args_of), GUESS>(args_of, eos, q);
 }

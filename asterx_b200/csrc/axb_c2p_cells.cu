@@ -42,7 +42,7 @@ AXB_D void run_solver_cells(int which, const EOS &eos, const C2PCellsArgs &a, Pr
 
 template <class EOS>
 __global__ void __launch_bounds__(128, AXB_C2P_MINB)
-    k_c2p_cells(const C2PCellsArgs a, const EOS eos) {
+    k_c2p_cells(const C2PCellsArgs a, const __grid_constant__ EOS eos) {
   __shared__ unsigned int s_hist[64];
   for (int q = threadIdx.x; q < 64; q += blockDim.x)
     s_hist[q] = 0;

@@ -34,7 +34,15 @@ struct EosIdeal {
     return gm1 * rho * eps;
   }
   // P / rho without the division (the root functions of the recovery)
-  AXB_HD double press_over_rho(double, double &eps, double) const { return gm1 * eps; }
+  // (`hint` is the tabulated EOS's)
+  AXB_HD double press_over_rho(double, double &eps, double, int &) const { return gm1 * eps; }
+  // press, temperature and entropy of a recovered state
+  AXB_HD void press_temp_entropy(double rho, double &eps, double ye, int, double &press,
+                                 double &temp, double &entropy) const {
+    press = press_from_valid_rho_eps_ye(rho, eps, ye);
+    temp = temp_from_valid_rho_eps_ye(rho, eps, ye);
+    entropy = kappa_from_valid_rho_eps_ye(rho, eps, ye);
+  }
   AXB_HD double eps_from_valid_rho_press_ye(double rho, double press, double) const {
     return press / (rho * gm1);
   }

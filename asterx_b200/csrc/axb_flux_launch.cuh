@@ -76,7 +76,7 @@ int launch_flux_pass_t(int dir, const RhsArgs &a, const axb_eos &eos,
 // batch with the grids of launch_flux_pass_eos).
 template <int DIR, int RECON, class EOS>
 __global__ void __launch_bounds__(128, AXB_FLUX_MINB)
-    k_flux_pass_batch(const RhsArgs *args, const TileTable t, unsigned long long *ctr, const EOS eos, const int seglen) {
+    k_flux_pass_batch(const RhsArgs *args, const TileTable t, unsigned long long *ctr, const __grid_constant__ EOS eos, const int seglen) {
   batch_loop(args, t, ctr, [&](const RhsArgs &a, const uint3 bid) {
     flux_pass_body<DIR, RECON, EOS>(a, eos, seglen, bid);
   });
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(128, AXB_FLUX_MINB)
 
 template <int RECON, class EOS>
 __global__ void __launch_bounds__(128, AXB_FLUX_X_MINB)
-    k_flux_x_batch(const RhsArgs *args, const TileTable t, unsigned long long *ctr, const EOS eos) {
+    k_flux_x_batch(const RhsArgs *args, const TileTable t, unsigned long long *ctr, const __grid_constant__ EOS eos) {
   batch_loop(args, t, ctr, [&](const RhsArgs &a, const uint3 bid) {
     flux_x_body<RECON, EOS>(a, eos, bid);
   });

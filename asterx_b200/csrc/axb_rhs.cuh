@@ -187,7 +187,14 @@ AXB_D void side_physics(const FaceMetric &m, const double *r, double Bdir,
   constexpr int D1 = (DIR + 1) % 3, D2 = (DIR + 2) % 3;
   const double rho = r[R_RHO], ent = r[R_ENT], ye = r[R_YE];
   double eps, press;
-  if (rec_temp) {
+  [[maybe_unused]] double tab_cs2, tab_eps;
+  if constexpr (EOS::kTabulated) { // always from the temperature (:297-304)
+    const auto th = eos.face_thermo(rho, r[R_PRESS], ye);
+    eps = th.eps;
+    press = th.press;
+    tab_cs2 = th.cs2;
+    tab_eps = th.eps2;
+  } else if (rec_temp) {
     eps = eos.eps_from_valid_rho_temp_ye(rho, r[R_PRESS], ye);
     press = eos.press_from_valid_rho_temp_ye(rho, r[R_PRESS], ye);
   } else {
@@ -256,15 +263,14 @@ AXB_D void side_physics(const FaceMetric &m, const double *r, double Bdir,
   // differ from the first
   double cs2, h;
   if constexpr (EOS::kTabulated) {
-    const double eps_in = eps;
-    const double cs = eos.csnd_from_valid_rho_eps_ye(rho, eps, ye);
-    cs2 = cs * (!(eps == eps_in) ? eos.csnd_from_valid_rho_eps_ye(rho, eps, ye) : cs);
-    h = 1 + eps + press / rho;
+    cs2 = tab_cs2;
+    h = 1 + tab_eps + press / rho;
   } else {
     // ideal gas: cs^2 without the square root, P/rho without the division
     // (last-ulp differences)
+    int hint = -1;
     cs2 = eos.csnd2_from_valid_rho_eps_ye(rho, eps, ye);
-    h = 1 + eps + eos.press_over_rho(rho, eps, ye);
+    h = 1 + eps + eos.press_over_rho(rho, eps, ye, hint);
   }
   const double dens = m.sqrtg * rho * W;
   const double DEnt = m.sqrtg * rho * W * ent;

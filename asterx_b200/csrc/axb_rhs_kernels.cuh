@@ -356,7 +356,7 @@ AXB_D void flux_pass_body(const RhsArgs &a, const EOS &eos, const int &seglen, c
 }
 template <int DIR, int RECON, class EOS, bool UCT = false>
 __global__ void __launch_bounds__(128, AXB_FLUX_MINB)
-    k_flux_pass(const RhsArgs a, const EOS eos, const int seglen) {
+    k_flux_pass(const RhsArgs a, const __grid_constant__ EOS eos, const int seglen) {
   flux_pass_body<DIR, RECON, EOS, UCT>(a, eos, seglen, blockIdx);
 }
 
@@ -432,7 +432,7 @@ AXB_D void flux_x_body(const RhsArgs &a, const EOS &eos, const uint3 bid) {
 }
 template <int RECON, class EOS, bool UCT = false>
 __global__ void __launch_bounds__(128, AXB_FLUX_X_MINB)
-    k_flux_x(const RhsArgs a, const EOS eos) {
+    k_flux_x(const RhsArgs a, const __grid_constant__ EOS eos) {
   flux_x_body<RECON, EOS, UCT>(a, eos, blockIdx);
 }
 

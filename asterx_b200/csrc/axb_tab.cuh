@@ -19,6 +19,13 @@
 
 namespace axb {
 
+// a query as a function call on the device (see EosTab::press_query)
+#ifdef __CUDACC__
+#define AXB_TAB_CALL __host__ __device__ __noinline__
+#else
+#define AXB_TAB_CALL
+#endif
+
 constexpr int TAB_NV = 4;
 enum { TAB_PRESS = 0, TAB_EPS = 1, TAB_S = 2, TAB_CS2 = 3 };
 // Iteration cap of the temperature root find.  The reference's loop has no
@@ -35,6 +42,10 @@ struct EosTab {
   const double *y; // TAB_NV values per node, node = i + n0*(j + n1*k)
   double shift;
   Range rgrho, rgye, rgtemp, rgeps;
+  // ln eps grows with T at every (rho, Ye) node by more than the rounding of
+  // its interpolation (set where the table is read): any search along T then
+  // finds the one cell that holds a value, so a query may start from a guess
+  int monotone;
   unsigned int *err; // status error word (device descriptor only), or null
 
   static constexpr bool kTabulated = true;
@@ -54,25 +65,43 @@ struct EosTab {
       return n[d] - 2;
     return static_cast<int>(t);
   }
-  AXB_HD static double lin(double A, double B, double xA, double xB, double xv) {
-    const double lam = (xv - xA) / (xB - xA);
-    return (B - A) * lam + A;
+  // The rho and Ye cells of a query and the weights in them, found once: all
+  // node values and interpolations of the query share them.
+  struct Cell {
+    int i, k;
+    double u, v;
+  };
+  AXB_HD Cell locate(double lrho, double ye) const {
+    Cell c;
+    c.i = find(0, lrho);
+    c.k = find(2, ye);
+    c.u = (lrho - x[0][c.i]) / (x[0][c.i + 1] - x[0][c.i]);
+    c.v = (ye - x[2][c.k]) / (x[2][c.k + 1] - x[2][c.k]);
+    return c;
   }
-  AXB_HD double interp(int var, double a, double b, double c) const {
-    const int i = find(0, a), j = find(1, b), k = find(2, c);
-    double Bk[2];
+  // linear in ln rho at temperature node j and Ye node c.k + o
+  AXB_HD double at_rho(int var, const Cell &c, int j, int o) const {
+    const double *p =
+        y + TAB_NV * (c.i + (long long)n[0] * (j + (long long)n[1] * (c.k + o))) + var;
+    const double y0 = p[0], y1 = p[TAB_NV];
+    return (y1 - y0) * c.u + y0;
+  }
+  // ln eps at temperature node j
+  AXB_HD double eps_node(const Cell &c, int j) const {
+    const double a = at_rho(TAB_EPS, c, j, 0), b = at_rho(TAB_EPS, c, j, 1);
+    return (b - a) * c.v + a;
+  }
+  // the trilinear interpolant, along ln rho, then ln T, then Ye
+  AXB_HD double tri(int var, const Cell &c, double lt) const {
+    const int j = find(1, lt);
+    const double w = (lt - x[1][j]) / (x[1][j + 1] - x[1][j]);
+    double B[2];
 #pragma unroll
-    for (int o2 = 0; o2 < 2; ++o2) {
-      double Aj[2];
-#pragma unroll
-      for (int o1 = 0; o1 < 2; ++o1) {
-        const long long base = i + (long long)n[0] * ((j + o1) + (long long)n[1] * (k + o2));
-        Aj[o1] = lin(y[TAB_NV * base + var], y[TAB_NV * (base + 1) + var], x[0][i],
-                     x[0][i + 1], a);
-      }
-      Bk[o2] = lin(Aj[0], Aj[1], x[1][j], x[1][j + 1], b);
+    for (int o = 0; o < 2; ++o) {
+      const double a = at_rho(var, c, j, o), b = at_rho(var, c, j + 1, o);
+      B[o] = (b - a) * w + a;
     }
-    return lin(Bk[0], Bk[1], x[2][k], x[2][k + 1], c);
+    return (B[1] - B[0]) * c.v + B[0];
   }
 
   template <class Fn>
@@ -143,14 +172,22 @@ struct EosTab {
     return sb;
   }
 
-  // logtemp_from_valid_rho_eps_ye (:197-228): clamps eps in place.
-  AXB_HD double logtemp(double rho, double &eps, double ye) const {
-    const double r = fmin(fmax(rho, rgrho.min), rgrho.max);
+  // logtemp_from_valid_rho_eps_ye (:197-228): clamps eps in place.  `c` is
+  // the cell of (ln of the clamped rho, Ye); `hint` a guess of the T cell
+  // (any value), replaced by the cell found.
+  AXB_HD double logtemp_at(const Cell &c, double lrho, double &eps, double ye, int &hint) const {
     eps = fmax(eps + shift, rgeps.min + shift) - shift;
-    const double lrho = log(r);
     const double leps = log(eps + shift);
-    const double vmin = interp(TAB_EPS, lrho, x0[1], ye);
-    const double vmax = interp(TAB_EPS, lrho, xlast[1], ye);
+    if (monotone && hint >= 1 && hint < n[1] - 2 && c.u >= 0.0 && c.u <= 1.0 && c.v >= 0.0 &&
+        c.v <= 1.0) {
+      // strictly inside the table (Ye is not clamped, so the weights are
+      // looked at) the bracketing cell is the search's result
+      const double e0 = eps_node(c, hint), e1 = eps_node(c, hint + 1);
+      if (e0 <= leps && leps < e1)
+        return in_cell(hint, leps, e0, e1);
+    }
+    const double vmin = tri(TAB_EPS, c, x0[1]);
+    const double vmax = tri(TAB_EPS, c, xlast[1]);
     if (leps <= vmin) {
       eps = exp(vmin) - shift;
       return x0[1];
@@ -159,7 +196,13 @@ struct EosTab {
       eps = exp(vmax) - shift;
       return xlast[1];
     }
-    return logtemp_root(lrho, leps, ye, vmin, vmax);
+    return logtemp_root(c, lrho, leps, ye, vmin, vmax, hint);
+  }
+  // the root of the linear equation in the T cell `j` with end values e0, e1
+  AXB_HD double in_cell(int j, double leps, double e0, double e1) const {
+    const double xa = x[1][j], xb = x[1][j + 1];
+    const double lam = fmin(fmax((leps - e0) / (e1 - e0), 0.0), 1.0);
+    return xa + lam * (xb - xa);
   }
 
   // The root in ln T of leps = interp(EPS, lrho, ln T, ye).  The
@@ -171,31 +214,16 @@ struct EosTab {
   // method on the whole axis to 1e-14 (eos_3p_tabulated3d.hxx:219-225,
   // eos_brent.hxx); both land on the same root of the same interpolant,
   // here to rounding.  Where the node values are not increasing around the
-  // root, the reference's Brent search is run instead.
-  AXB_HD double logtemp_root(double lrho, double leps, double ye, double vlo, double vhi) const {
+  // root, the reference's Brent search is run instead.  The bisection
+  // evaluates the interpolant at temperature nodes, where it is the bilinear
+  // interpolant in (ln rho, Ye) of that node's four values.
+  AXB_HD double logtemp_root(const Cell &c, double lrho, double leps, double ye, double vlo,
+                             double vhi, int &hint) const {
     // vlo = interp at node 0 < leps < vhi = interp at the last node.
-    // The bisection evaluates the interpolant at temperature nodes, where it
-    // is the bilinear interpolant in (ln rho, Ye) of that node's four
-    // values: the rho and Ye cells and weights are found once, and each step
-    // reads four values (interp's own arithmetic with the temperature weight
-    // zero)
-    const int i = find(0, lrho), k = find(2, ye);
-    const double lam_r = (lrho - x[0][i]) / (x[0][i + 1] - x[0][i]);
-    const double lam_y = (ye - x[2][k]) / (x[2][k + 1] - x[2][k]);
-    auto at_node = [&](int jn) {
-      double A[2];
-#pragma unroll
-      for (int o2 = 0; o2 < 2; ++o2) {
-        const long long base = i + (long long)n[0] * (jn + (long long)n[1] * (k + o2));
-        const double y0 = y[TAB_NV * base + TAB_EPS], y1 = y[TAB_NV * (base + 1) + TAB_EPS];
-        A[o2] = (y1 - y0) * lam_r + y0;
-      }
-      return (A[1] - A[0]) * lam_y + A[0];
-    };
     int lo = 0, hi = n[1] - 1;
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
-      const double vm = at_node(mid);
+      const double vm = eps_node(c, mid);
       if (vm <= leps) {
         lo = mid;
         vlo = vm;
@@ -204,33 +232,20 @@ struct EosTab {
         vhi = vm;
       }
     }
-    // the cell [x_lo, x_lo+1]: interp = c0 + c1 * lambda, lambda in [0, 1]
-    const double xa = x[1][lo], xb = x[1][lo + 1];
-    double c[2][2]; // [T end][Ye end] after the interpolation along ln rho
-#pragma unroll
-    for (int o2 = 0; o2 < 2; ++o2)
-#pragma unroll
-      for (int o1 = 0; o1 < 2; ++o1) {
-        const long long base =
-            i + (long long)n[0] * ((lo + o1) + (long long)n[1] * (k + o2));
-        const double y0 = y[TAB_NV * base + TAB_EPS], y1 = y[TAB_NV * (base + 1) + TAB_EPS];
-        c[o1][o2] = (y1 - y0) * lam_r + y0; // lin along ln rho, its weight found once
-      }
-    const double e0 = (c[0][1] - c[0][0]) * lam_y + c[0][0]; // at x_lo
-    const double e1 = (c[1][1] - c[1][0]) * lam_y + c[1][0]; // at x_lo+1
+    hint = lo;
+    // the cell [x_lo, x_lo+1]: interp = e0 + (e1 - e0) * lambda, lambda in [0, 1]
+    const double e0 = eps_node(c, lo), e1 = eps_node(c, lo + 1);
     if (!(vlo <= leps && leps <= vhi) || !(e1 > e0)) {
       bool capped;
       const double lt = zero_brent(
-          x0[1], xlast[1], 1.e-14,
-          [&](double l) { return leps - interp(TAB_EPS, lrho, l, ye); }, capped);
+          x0[1], xlast[1], 1.e-14, [&](double l) { return leps - tri(TAB_EPS, c, l); }, capped);
 #ifdef __CUDA_ARCH__
       if (capped && err)
         atomicOr(err, AXB_EW_ROOT_CAP);
 #endif
       return lt;
     }
-    const double lam = fmin(fmax((leps - e0) / (e1 - e0), 0.0), 1.0);
-    return xa + lam * (xb - xa);
+    return in_cell(lo, leps, e0, e1);
   }
   AXB_HD double lr_clamped(double rho) const {
     return log(fmin(fmax(rho, rgrho.min), rgrho.max));
@@ -238,13 +253,67 @@ struct EosTab {
   AXB_HD double lt_clamped(double temp) const {
     return log(fmin(fmax(temp, rgtemp.min), rgtemp.max));
   }
-  AXB_HD double press_over_rho(double rho, double &eps, double ye) const {
-    return press_from_valid_rho_eps_ye(rho, eps, ye) / rho;
+  // The queries are function calls, not inlined: a recovery evaluates them
+  // at a dozen places, and inlined the kernel did not fit the instruction
+  // cache (16 of its 55 stalled cycles per issued instruction were fetches).
+  struct Query {
+    double value, eps; // eps as the query leaves it
+    int hint;
+  };
+  AXB_TAB_CALL Query press_query(double rho, double eps, double ye, int hint) const {
+    Query q{0.0, eps, hint};
+    const double lr = lr_clamped(rho);
+    const Cell c = locate(lr, ye);
+    const double lt = logtemp_at(c, lr, q.eps, ye, q.hint);
+    q.value = exp(tri(TAB_PRESS, c, lt));
+    return q;
+  }
+  AXB_TAB_CALL Query logtemp_query(double rho, double eps, double ye, int hint) const {
+    Query q{0.0, eps, hint};
+    const double lr = lr_clamped(rho);
+    q.value = logtemp_at(locate(lr, ye), lr, q.eps, ye, q.hint);
+    return q;
+  }
+  AXB_TAB_CALL double interp(int var, double lrho, double lt, double ye) const {
+    return tri(var, locate(lrho, ye), lt);
+  }
+  // eps, press and the product of two sound-speed queries of a face state
+  // given by its temperature (fluxes.cxx:297-304,556-560): eps from the
+  // clamped logarithms, press from the plain ones, as the two queries take
+  // them; cs^2 at that eps, found from the temperature's own cell.  eps2 is
+  // eps as the sound-speed query leaves it (it may clamp).
+  struct FaceThermo {
+    double eps, press, cs2, eps2;
+  };
+  AXB_TAB_CALL FaceThermo face_thermo(double rho, double temp, double ye) const {
+    FaceThermo o;
+    const double r = fmin(fmax(rho, rgrho.min), rgrho.max);
+    const double T = fmin(fmax(temp, rgtemp.min), rgtemp.max);
+    const double lr = log(r), lt = log(T);
+    const Cell c = locate(lr, ye);
+    o.eps = exp(tri(TAB_EPS, c, lt)) - shift;
+    if (r == rho && T == temp)
+      o.press = exp(tri(TAB_PRESS, c, lt));
+    else
+      o.press = exp(tri(TAB_PRESS, locate(log(rho), ye), log(temp)));
+    o.eps2 = o.eps;
+    int hint = find(1, lt);
+    const double cs = sqrt(tri(TAB_CS2, c, logtemp_at(c, lr, o.eps2, ye, hint)));
+    o.cs2 = cs * cs;
+    if (!(o.eps2 == o.eps))
+      o.cs2 = cs * sqrt(tri(TAB_CS2, c, logtemp_at(c, lr, o.eps2, ye, hint)));
+    return o;
+  }
+  AXB_HD double press_over_rho(double rho, double &eps, double ye, int &hint) const {
+    const Query q = press_query(rho, eps, ye, hint);
+    eps = q.eps;
+    hint = q.hint;
+    return q.value / rho;
   }
   AXB_HD double press_from_valid_rho_eps_ye(double rho, double &eps, double ye) const {
-    const double lr = lr_clamped(rho);
-    const double lt = logtemp(rho, eps, ye);
-    return exp(interp(TAB_PRESS, lr, lt, ye));
+    const Query q = press_query(rho, eps, ye, -1);
+    eps = q.eps;
+    return q.value;
   }
   // takes the logs of the unclamped inputs, as the reference does (:230-239)
   AXB_HD double press_from_valid_rho_temp_ye(double rho, double temp, double ye) const {
@@ -259,13 +328,32 @@ struct EosTab {
   // limit (v_lim, the table's largest rho, the pressure atmosphere) fires
   // with use_temperature off
   AXB_HD double eps_from_valid_rho_press_ye(double, double, double) const { return 0.0; }
+  AXB_HD double logtemp(double rho, double &eps, double ye) const {
+    const Query q = logtemp_query(rho, eps, ye, -1);
+    eps = q.eps;
+    return q.value;
+  }
   AXB_HD double csnd_from_valid_rho_eps_ye(double rho, double &eps, double ye) const {
-    const double lr = lr_clamped(rho);
     const double lt = logtemp(rho, eps, ye);
-    return sqrt(interp(TAB_CS2, lr, lt, ye));
+    return sqrt(interp(TAB_CS2, lr_clamped(rho), lt, ye));
   }
   AXB_HD double temp_from_valid_rho_eps_ye(double rho, double &eps, double ye) const {
     return exp(logtemp(rho, eps, ye));
+  }
+  // press, temperature and entropy of a recovered state, one after another
+  // (each may clamp eps, as the separate queries do); `hint` as above
+  AXB_HD void press_temp_entropy(double rho, double &eps, double ye, int hint, double &press,
+                                 double &temp, double &entropy) const {
+    const Query p = press_query(rho, eps, ye, hint);
+    press = p.value;
+    Query q = logtemp_query(rho, p.eps, ye, p.hint);
+    temp = exp(q.value);
+    // kappa_from_valid_rho_eps_ye inverts once more: the same inversion
+    // unless the last one moved eps
+    if (!(q.eps == p.eps))
+      q = logtemp_query(rho, q.eps, ye, q.hint);
+    eps = q.eps;
+    entropy = entropy_from_valid_rho_temp_ye(rho, exp(q.value), ye);
   }
   AXB_HD double entropy_from_valid_rho_temp_ye(double rho, double temp, double ye) const {
     return interp(TAB_S, lr_clamped(rho), lt_clamped(temp), ye);
