@@ -364,6 +364,71 @@ AXB_HD void set_E(Prim &pv, const sym3 &gup) {
   lower3(gup, El, pv.E);
 }
 
+// The Newton search of the Noble scheme (c2p_2DNoble.hxx:404-515) in (Z, v^2)
+// from undensitised D, E = tau + D, S^2, B^2 and B.S; gg = (Gamma-1)/Gamma.
+// A step takes two divisions and one reciprocal square root where the
+// reference's expressions take seven divisions and a square root (FP64
+// divisions were most of a step's time): the divisions by Gamma become one
+// product with gg, sqrt(1-v^2) and its reciprocal come from one rsqrt, the
+// determinant is formed from the Jacobian's terms, |dx/x| <= tol is tested as
+// |dx| <= tol |x|, and multiply-adds are explicit.  Last-ulp differences in a
+// search that converges quadratically to tol.
+struct NobleRoot {
+  double Z, vsq;
+  int iters;
+  bool slow;   // not converged within max_iter
+  bool finite; // the last residual is finite
+};
+AXB_HD NobleRoot noble_root(double D, double E, double Ssq, double Bsq, double BiSi, double gg,
+                            double Zmin, double tol, int max_iter, double x0, double x1) {
+  constexpr double dv = (1. - 1.e-10);
+  const double b2 = BiSi * BiSi, hB = 0.5 * Bsq;
+  double xo0 = x0, err = 1.0, lim = 0.0, r0 = 0.0, r1 = 0.0;
+  if (x1 < 0.0)
+    x1 = 0.0;
+  else if (x1 >= 1.0)
+    x1 = dv;
+  if (x0 <= 0.0)
+    x0 = fabs(x0) + Zmin;
+  else if (x0 > 1e20)
+    x0 = xo0;
+  int k;
+  for (k = 1; k <= max_iter; ++k) {
+    const double Z = x0, V = x1;
+    const double iZ = 1.0 / Z;
+    const double om = 1.0 - V;
+    const double is = rsqrt(om);
+    const double ZB = Bsq + Z, ZB2 = ZB * ZB;
+    const double b2z2 = b2 * iZ * iZ, Vb = fma(b2z2, iZ, V); // v^2 + (B.S)^2 / Z^3
+    const double p = fma(Z, om, -D * (om * is)) * gg;        // P(Z, v^2)
+    const double dPv = fma(0.5 * D, is, -Z) * gg;
+    const double fj00 = -2.0 * Vb * ZB;
+    const double fj10 = fma(om, gg, -1.0) - (Vb - V);
+    const double fj11 = dPv - hB;
+    r0 = fma(b2z2, ZB + Z, fma(-V, ZB2, Ssq));
+    r1 = (fma(0.5, b2z2, fma(-hB, 1.0 + V, E)) - Z) + p;
+    const double idet = 1.0 / fma(fj10, ZB2, fj00 * fj11);
+    const double dx0 = -fma(fj11, r0, ZB2 * r1) * idet;
+    const double dx1 = -fma(-fj10, r0, fj00 * r1) * idet;
+    xo0 = x0;
+    x0 += dx0;
+    x1 += dx1;
+    if (x1 < 0.0)
+      x1 = 0.0;
+    else if (x1 >= 1.0)
+      x1 = dv;
+    if (x0 <= 0.0)
+      x0 = fabs(x0) + Zmin;
+    else if (x0 > 1e20)
+      x0 = xo0;
+    err = fabs(dx0);
+    lim = x0 == 0.0 ? tol : tol * fabs(x0);
+    if (err <= lim)
+      break;
+  }
+  return {x0, x1, k, err > lim, isfinite(r0 * r0 + r1 * r1)};
+}
+
 // ---------------------------------------------------------------------------
 // Noble 2D (c2p_2DNoble::solve, c2p_2DNoble.hxx:275-594).  The ideal-gas
 // pressure P(Z, v^2) = (Z(1-v^2) - D sqrt(1-v^2)) (Gamma-1)/Gamma closes the
@@ -442,70 +507,19 @@ AXB_HD void noble_solve(const EOS &eos, const C2PParams &cp, const Atmo &atmo,
     x0 = zguess;
     x1 = vsqguess;
   }
-  double xo0 = x0;
-  constexpr double dv = (1. - 1.e-10);
-  double errx = 1., df = 1., f = 1.;
-  if (x1 < 0.0)
-    x1 = 0.0;
-  else if (x1 >= 1.0)
-    x1 = dv;
-  if (x0 <= 0.0)
-    x0 = fabs(x0) + Zmin;
-  else if (x0 > 1e20)
-    x0 = xo0;
-  const double gfac = (gamma - 1.0);
-  int k;
-  for (k = 1; k <= cp.maxIter; k++) {
-    const double Z = x0;
-    const double invZ = 1.0 / Z;
-    const double Vsq = x1;
-    const double Sdotn = -(cv.tau + cv.dens);
-    const double p_tmp = ((Z * (1.0 - Vsq) - cv.dens * sqrt(1.0 - Vsq)) * gfac / (gamma));
-    const double dPdvsq = ((-Z + cv.dens / (2.0 * sqrt(1.0 - Vsq))) * gfac / gamma);
-    const double dPdZ = ((1.0 - Vsq) * gfac / gamma);
-    const double fj00 = -2 * (Vsq + BiSi * BiSi * invZ * invZ * invZ) * (Bsq + Z);
-    const double fj01 = -(Bsq + Z) * (Bsq + Z);
-    const double fj10 = -1.0 + dPdZ - BiSi * BiSi * invZ * invZ * invZ;
-    const double fj11 = -0.5 * Bsq + dPdvsq;
-    const double r0 = Ssq - Vsq * (Bsq + Z) * (Bsq + Z) +
-                      BiSi * BiSi * invZ * invZ * (Bsq + Z + Z);
-    const double r1 = -Sdotn - 0.5 * Bsq * (1.0 + Vsq) +
-                      0.5 * BiSi * BiSi * invZ * invZ - Z + p_tmp;
-    const double detjac =
-        (Bsq + Z) * (fj10 * (Bsq + Z) +
-                     (Bsq - 2.0 * dPdvsq) * (BiSi * BiSi * invZ * invZ + Vsq * Z) * invZ);
-    const double detjac_inv = 1.0 / detjac;
-    const double dx0 = -(fj11 * r0 - fj01 * r1) * detjac_inv;
-    const double dx1 = -(-fj10 * r0 + fj00 * r1) * detjac_inv;
-    df = -r0 * r0 - r1 * r1;
-    f = -0.5 * (df);
-    errx = 0.;
-    xo0 = x0;
-    x0 += dx0;
-    x1 += dx1;
-    if (x1 < 0.0)
-      x1 = 0.0;
-    else if (x1 >= 1.0)
-      x1 = dv;
-    if (x0 <= 0.0)
-      x0 = fabs(x0) + Zmin;
-    else if (x0 > 1e20)
-      x0 = xo0;
-    errx = (x0 == 0.) ? fabs(dx0) : fabs(dx0 / x0);
-    if (fabs(errx) <= cp.tol)
-      break;
-  }
-  rep.iters = k;
-  if (fabs(errx) > cp.tol) {
+  const NobleRoot root = noble_root(cv.dens, cv.tau + cv.dens, Ssq, Bsq, BiSi,
+                                    (gamma - 1.0) / gamma, Zmin, cp.tol, cp.maxIter, x0, x1);
+  rep.iters = root.iters;
+  if (root.slow) {
     rep.fail(REP_ROOT_FAIL_CONV);
     cv.scale(sqrt_detg);
     return;
   }
-  if (!isfinite(f) || !isfinite(df))
+  if (!root.finite)
     rep.fail(REP_ROOT_FAIL_BRACKET);
   // WZ2Prim (c2p_2DNoble.hxx:192-273)
   {
-    const double Z_Sol = x0, vsq_Sol = x1;
+    const double Z_Sol = root.Z, vsq_Sol = root.vsq;
     const double W_Sol = 1.0 / sqrt(1.0 - vsq_Sol);
     pv.rho = cv.dens / W_Sol;
     vel_from_Z(Z_Sol, W_Sol, Bsq, BiSi, cp.use_zprim, pv, cv, gup, glo);

@@ -20,7 +20,7 @@ struct C2PCellsArgs {
   C2PParams cp;
   int c2p_prime, c2p_second, use_entropy_fix;
   Atmo atmo;
-  double gamma_noble, Zmin;
+  double gamma_noble, Zmin, gfac_over_gamma;
   int use_mlp;
   double bracket;
   MlpDev mlp;
@@ -40,19 +40,58 @@ AXB_D void run_solver_cells(int which, const EOS &eos, const C2PCellsArgs &a, Pr
     entropy_solve(eos, a.cp, a.atmo, pv, cv, glo, rep);
 }
 
-template <class EOS>
-__global__ void __launch_bounds__(128, AXB_C2P_MINB)
-    k_c2p_cells(const C2PCellsArgs a, const __grid_constant__ EOS eos) {
-  __shared__ unsigned int s_hist[64];
-  for (int q = threadIdx.x; q < 64; q += blockDim.x)
-    s_hist[q] = 0;
+// A cell's outputs; any pointer may be null.
+AXB_D void c2p_cells_store(const axb_cells &c, long long i, int code, int iters_first,
+                           bool fallback, const Prim &pv) {
+  if (c.flag)
+    c.flag[i] = code;
+  if (c.fallback)
+    c.fallback[i] = fallback ? 1.0 : 0.0;
+  if (c.iters)
+    c.iters[i] = iters_first;
+  if (c.rho)
+    c.rho[i] = pv.rho;
+  if (c.eps)
+    c.eps[i] = pv.eps;
+  if (c.press)
+    c.press[i] = pv.press;
+  for (int q = 0; q < 3; ++q)
+    if (c.vel[q])
+      c.vel[q][i] = pv.vel[q];
+  if (c.w_lorentz)
+    c.w_lorentz[i] = pv.w_lor;
+  if (c.Ye)
+    c.Ye[i] = pv.Ye;
+  if (c.temperature)
+    c.temperature[i] = pv.temperature;
+  if (c.entropy)
+    c.entropy[i] = pv.entropy;
+}
+
+// Failure count and iteration histogram (every thread of the block arrives).
+AXB_D void c2p_cells_epilogue(const C2PCellsArgs &a, unsigned int *s_hist, int iters_first,
+                              bool failed) {
+  const unsigned nfail = __popc(__ballot_sync(0xffffffffu, failed));
+  if (nfail && (threadIdx.x % 32) == 0) {
+    atomicAdd(&a.status->c2p_fail_count, nfail);
+    atomicOr(&a.status->error_word, AXB_EW_C2P_FAIL);
+  }
+  if (iters_first >= 0)
+    atomicAdd(&s_hist[min(iters_first, 63)], 1u);
   __syncthreads();
+  for (int q = threadIdx.x; q < 64; q += blockDim.x)
+    if (s_hist[q])
+      atomicAdd(&a.status->c2p_iter_hist[q], (unsigned long long)s_hist[q]);
+}
+
+// The whole cascade on cell i.
+template <class EOS>
+AXB_D void c2p_cells_one(const C2PCellsArgs &a, const EOS &eos, const long long i,
+                         int &iters_first, bool &failed) {
   const axb_cells &c = a.c;
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = i < c.n;
   Cons cv;
-  sym3 glo{1, 0, 0, 1, 0, 1};
-  if (valid) {
+  sym3 glo;
+  {
     cv.dens = c.dens[i];
     for (int q = 0; q < 3; ++q) {
       cv.mom[q] = c.mom[q][i];
@@ -65,7 +104,7 @@ __global__ void __launch_bounds__(128, AXB_C2P_MINB)
   }
   // learned guess (x = h W, W) from k_mlp_guess_tc
   double zguess = -1.0, vsqguess = -1.0, xlo = -1.0, xhi = -1.0;
-  if (a.use_mlp && valid) {
+  if (a.use_mlp) {
     const float2 gs = reinterpret_cast<const float2 *>(c.guess)[i];
     const double x = gs.x, W = gs.y;
     zguess = cv.dens / sqrt(det3(glo)) * x; // Z = rho h W^2 = D (h W)
@@ -75,9 +114,8 @@ __global__ void __launch_bounds__(128, AXB_C2P_MINB)
     if (!(zguess > 0.0 && zguess < 1e300 && vsqguess >= 0.0 && vsqguess < 1.0))
       zguess = vsqguess = xlo = xhi = -1.0;
   }
-  int iters_first = -1;
-  bool failed = false, fallback = false;
-  if (valid) {
+  bool fallback = false;
+  {
     const double sqrt_detg = sqrt(det3(glo));
     const double isg = 1.0 / sqrt_detg;
     const double Bup[3] = {cv.dBvec[0] * isg, cv.dBvec[1] * isg, cv.dBvec[2] * isg};
@@ -173,41 +211,174 @@ __global__ void __launch_bounds__(128, AXB_C2P_MINB)
         a.atmo.set(pv, cv, glo);
       }
     }
-    if (c.flag)
-      c.flag[i] = code;
-    if (c.fallback)
-      c.fallback[i] = fallback ? 1.0 : 0.0;
-    if (c.iters)
-      c.iters[i] = iters_first;
-    if (c.rho)
-      c.rho[i] = pv.rho;
-    if (c.eps)
-      c.eps[i] = pv.eps;
-    if (c.press)
-      c.press[i] = pv.press;
-    for (int q = 0; q < 3; ++q)
-      if (c.vel[q])
-        c.vel[q][i] = pv.vel[q];
-    if (c.w_lorentz)
-      c.w_lorentz[i] = pv.w_lor;
-    if (c.Ye)
-      c.Ye[i] = pv.Ye;
-    if (c.temperature)
-      c.temperature[i] = pv.temperature;
-    if (c.entropy)
-      c.entropy[i] = pv.entropy;
+    c2p_cells_store(c, i, code, iters_first, fallback, pv);
   }
-  const unsigned nfail = __popc(__ballot_sync(0xffffffffu, failed));
-  if (nfail && (threadIdx.x % 32) == 0) {
-    atomicAdd(&a.status->c2p_fail_count, nfail);
-    atomicOr(&a.status->error_word, AXB_EW_C2P_FAIL);
-  }
-  if (iters_first >= 0)
-    atomicAdd(&s_hist[min(iters_first, 63)], 1u);
-  __syncthreads();
+}
+
+template <class EOS>
+__global__ void __launch_bounds__(128, AXB_C2P_MINB)
+    k_c2p_cells(const C2PCellsArgs a, const __grid_constant__ EOS eos) {
+  __shared__ unsigned int s_hist[64];
   for (int q = threadIdx.x; q < 64; q += blockDim.x)
-    if (s_hist[q])
-      atomicAdd(&a.status->c2p_iter_hist[q], (unsigned long long)s_hist[q]);
+    s_hist[q] = 0;
+  __syncthreads();
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  int iters_first = -1;
+  bool failed = false;
+  if (i < a.c.n)
+    c2p_cells_one(a, eos, i, iters_first, failed);
+  c2p_cells_epilogue(a, s_hist, iters_first, failed);
+}
+
+// ---------------------------------------------------------------------------
+// The fast form for the ideal gas with Noble first: only the first solver's
+// common path, so that it fits 8 CTAs per SM where the whole cascade takes the
+// registers of 4, and without what the cascade's general form repeats (a
+// cell's metric determinant, its inverse and root once; no conserved
+// variables to rebuild).  Any cell that needs more -- an invalid metric,
+// non-finite or over-magnetised conserved variables, a Newton search that
+// does not converge, a non-positive rho or eps -- calls the cascade of
+// k_c2p_cells, out of line, having written nothing.
+//
+// With noble_root's cheaper step, 4.0M cells: plain 1156 -> 445 us, learned
+// (recovery alone) 691 -> 297 us.
+// ---------------------------------------------------------------------------
+__device__ __noinline__ void c2p_cells_cascade(const C2PCellsArgs &a, const EosIdeal &eos,
+                                               long long i, int &iters_first, bool &failed) {
+  c2p_cells_one(a, eos, i, iters_first, failed);
+}
+
+__global__ void __launch_bounds__(128, 8)
+    k_c2p_cells_noble(const __grid_constant__ C2PCellsArgs a,
+                      const __grid_constant__ EosIdeal eos) {
+  __shared__ unsigned int s_hist[64];
+  for (int q = threadIdx.x; q < 64; q += blockDim.x)
+    s_hist[q] = 0;
+  __syncthreads();
+  const axb_cells &c = a.c;
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  int iters_first = -1;
+  bool failed = false;
+  if (i < c.n) {
+    const sym3 g{c.g[0][i], c.g[1][i], c.g[2][i], c.g[3][i], c.g[4][i], c.g[5][i]};
+    const double det = det3(g);
+    const double isg = rsqrt(det);
+    const double idet = isg * isg;
+    const double D = c.dens[i] * isg;
+    double S[3], B[3];
+    for (int q = 0; q < 3; ++q) {
+      S[q] = c.mom[q][i] * isg;
+      B[q] = c.dB[q][i] * isg;
+    }
+    double tau = c.tau[i] * isg;
+    const double DYe = c.DYe[i] * isg;
+    const double DEnt = c.DEnt ? c.DEnt[i] : 0.0;
+    double Bl[3], Sup[3];
+    lower3(g, B, Bl);
+    const double Bsq = dot3(Bl, B);
+    sym3 u; // the inverse metric
+    u.xx = (g.yy * g.zz - g.yz * g.yz) * idet;
+    u.xy = (g.xz * g.yz - g.xy * g.zz) * idet;
+    u.xz = (g.xy * g.yz - g.xz * g.yy) * idet;
+    u.yy = (g.xx * g.zz - g.xz * g.xz) * idet;
+    u.yz = (g.xy * g.xz - g.xx * g.yz) * idet;
+    u.zz = (g.xx * g.yy - g.xy * g.xy) * idet;
+    lower3(u, S, Sup);
+    double Ssq = dot3(S, Sup);
+    // cons_floors_and_ceilings (c2p.hxx:330-369), undensitised
+    const double tau_lim = 0.5 * Bsq;
+    if (tau <= tau_lim)
+      tau = tau_lim;
+    const double slim = D + tau;
+    if (Ssq > slim * slim) {
+      const double f = sqrt(slim * slim / Ssq);
+      for (int q = 0; q < 3; ++q) {
+        S[q] *= f;
+        Sup[q] *= f;
+      }
+      Ssq = Ssq * (f * f);
+    }
+    const double BiSi = dot3(S, B);
+    const bool atmosphere = D <= a.atmo.rho_cut;
+    bool common = g.xx > 0.0 && g.xx * g.yy - g.xy * g.xy > 0.0 && det > 0.0 && isfinite(D) &&
+                  isfinite(Ssq) && isfinite(Bsq) && isfinite(BiSi) && isfinite(DYe) &&
+                  isfinite(DEnt) && !(Bsq > a.cp.Bsq_lim);
+    Prim pv;
+    int code = AXB_C2P_PRIME;
+    if (common && atmosphere) {
+      a.atmo.set(pv);
+      code = AXB_C2P_ATMO;
+    } else if (common) {
+      // start: the learned guess, or the seeds' (Z, v^2)
+      double x0 = -1.0, x1 = -1.0;
+      if (a.use_mlp) {
+        const float2 gs = reinterpret_cast<const float2 *>(c.guess)[i];
+        const double x = gs.x, W = gs.y;
+        x0 = D * x; // Z = rho h W^2 = D (h W)
+        x1 = 1.0 - 1.0 / (W * W);
+        if (!(x0 > 0.0 && x0 < 1e300 && x1 >= 0.0 && x1 < 1.0))
+          x0 = x1 = -1.0;
+      }
+      if (!(x0 >= 0.0)) {
+        double eps = a.atmo.eps, vsq = 0.0;
+        if (c.seed_rho) {
+          double v[3], vl[3];
+          for (int q = 0; q < 3; ++q)
+            v[q] = c.seed_vel[q][i];
+          lower3(g, v, vl);
+          vsq = dot3(vl, v);
+          if (vsq >= 1.0) // limited to v_lim, as con2prim.cxx:168-209
+            vsq = a.cp.v_lim * a.cp.v_lim;
+          eps = fmax(c.seed_eps[i], a.atmo.eps);
+        }
+        // rho = D / W, Z = (rho + eps rho + P) W^2 = D W (1 + eps + P/rho)
+        const double W = rsqrt(1.0 - vsq);
+        x0 = fabs(D * W * (1.0 + eps + eos.gm1 * eps));
+        x1 = vsq;
+      }
+      const NobleRoot r = noble_root(D, tau + D, Ssq, Bsq, BiSi, a.gfac_over_gamma, a.Zmin,
+                                     a.cp.tol, a.cp.maxIter, x0, x1);
+      common = !r.slow && r.finite;
+      if (common) {
+        // WZ2Prim (c2p_2DNoble.hxx:192-273): W = (1 - v^2)^-1/2, rho = D / W,
+        // eps = (Z / (W^2 rho) - 1) / Gamma = (Z / (W D) - 1) / Gamma
+        const double om = 1.0 - r.vsq;
+        const double W = rsqrt(om);
+        const double iW = om * W;
+        const double iD = 1.0 / D;
+        pv.rho = D * iW;
+        pv.w_lor = W;
+        const double iZZB = 1.0 / (r.Z * (r.Z + Bsq));
+        const double iZB = r.Z * iZZB;
+        for (int q = 0; q < 3; ++q)
+          pv.vel[q] = fma(BiSi * iZZB, B[q], Sup[q] * iZB);
+        pv.eps = fma(r.Z * iW, iD, -1.0) * eos.inv_gamma;
+        pv.Ye = DYe * iD;
+        common = pv.rho > 0.0 && pv.eps > 0.0;
+        if (common) {
+          pv.press = eos.press_from_valid_rho_eps_ye(pv.rho, pv.eps, pv.Ye);
+          pv.temperature = eos.temp_from_valid_rho_eps_ye(pv.rho, pv.eps, pv.Ye);
+          pv.entropy = eos.kappa_from_valid_rho_eps_ye(pv.rho, pv.eps, pv.Ye);
+          iters_first = r.iters;
+          if (pv.rho < a.atmo.rho_cut) {
+            a.atmo.set(pv);
+          } else {
+            Report rep;
+            Cons cv;
+            cv.dens = D;
+            prims_floors(eos, a.cp, a.atmo, pv, cv, g, rep);
+          }
+        }
+      }
+    }
+    if (common) {
+      c2p_cells_store(c, i, code, iters_first, false, pv);
+    } else {
+      iters_first = -1;
+      c2p_cells_cascade(a, eos, i, iters_first, failed);
+    }
+  }
+  c2p_cells_epilogue(a, s_hist, iters_first, failed);
 }
 } // namespace axb
 
@@ -268,12 +439,13 @@ AXB_API int axb_c2p_cells(axb_ctx *ctx, const axb_cells *cells, const axb_params
   hb.poly = eos->poly;
   if (eos->kind == 0) {
     a.gamma_noble = eos->ideal.gamma;
+    a.gfac_over_gamma = (a.gamma_noble - 1.0) / a.gamma_noble;
     a.Zmin = eos->ideal.rgrho.min;
     a.atmo = host_atmosphere(hb, eos->ideal);
   } else if (eos->kind == 1) {
     if (p->thermal_eos_atmo && p->use_press_atmo)
       return AXB_ERR_UNSUPPORTED;
-    a.gamma_noble = std::numeric_limits<double>::quiet_NaN();
+    a.gamma_noble = a.gfac_over_gamma = std::numeric_limits<double>::quiet_NaN();
     a.Zmin = eos->tab_h.rgrho.min;
     a.atmo = host_atmosphere(hb, eos->tab_h);
   } else {
@@ -296,6 +468,8 @@ AXB_API int axb_c2p_cells(axb_ctx *ctx, const axb_cells *cells, const axb_params
   axb_mark(ctx, AXB_R_C2P_CELLS, s, true);
   if (eos->kind == 1)
     k_c2p_cells<<<(unsigned)blocks, 128, 0, s>>>(a, tab_for_launch(*eos, a.status));
+  else if (a.c2p_prime == AXB_C2P_NOBLE && !a.cp.use_zprim)
+    k_c2p_cells_noble<<<(unsigned)blocks, 128, 0, s>>>(a, eos->ideal);
   else
     k_c2p_cells<<<(unsigned)blocks, 128, 0, s>>>(a, eos->ideal);
   axb_mark(ctx, AXB_R_C2P_CELLS, s, false);
