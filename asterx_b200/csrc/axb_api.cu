@@ -964,7 +964,7 @@ uint3 flux_grid(int dir, const axb_box &b, int seglen) {
   }
   const int T1 = dir == 2 ? 1 : 2;
   const long long plane = (long long)(b.n[0] + 2) * (b.n[T1] + 2);
-  return make_uint3(unsigned((plane + 127) / 128), 1, (b.n[dir] + seglen - 1) / seglen);
+  return make_uint3(unsigned((plane + FLUX_T - 1) / FLUX_T), 1, (b.n[dir] + seglen - 1) / seglen);
 }
 } // namespace axb
 

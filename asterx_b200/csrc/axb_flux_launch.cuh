@@ -8,6 +8,13 @@
 
 namespace axb {
 
+// a y or z pass, with its dynamic shared memory allowed
+template <class K, class... Args>
+void launch_pass(K kernel, dim3 grid, dim3 block, cudaStream_t s, const Args &...args) {
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FLUX_SMEM);
+  kernel<<<grid, block, FLUX_SMEM, s>>>(args...);
+}
+
 template <int RECON, class EOS, bool UCT>
 int launch_flux_pass_uct(int dir, const RhsArgs &a, const EOS &eos, int seglen,
                          cudaStream_t s) {
@@ -22,7 +29,7 @@ int launch_flux_pass_uct(int dir, const RhsArgs &a, const EOS &eos, int seglen,
     return cudaGetLastError() == cudaSuccess ? AXB_OK : AXB_ERR_CUDA;
   }
   const int T0 = 0, T1 = dir == 2 ? 1 : 2;
-  const dim3 block(32, 4);
+  const dim3 block(32, FLUX_T / 32);
   // Thread layout: 32 columns x 4 rows of the transverse plane per block,
   // or the plane walked row after row (no lane idle on the n+2-wide rows).
   // Measured at 256^3: the packed walk is 7-9 % faster for WENO-Z and PPM,
@@ -30,12 +37,12 @@ int launch_flux_pass_uct(int dir, const RhsArgs &a, const EOS &eos, int seglen,
   // share the face metric's second vertex row in L1).
   constexpr bool packed = RECON != AXB_RECON_MP5;
   if (!packed) {
-    const dim3 grid((b.n[T0] + 2 * a.text + 31) / 32, (b.n[T1] + 2 * a.text + 3) / 4,
+    const dim3 grid((b.n[T0] + 2 * a.text + 31) / 32, (b.n[T1] + 2 * a.text + FLUX_T / 32 - 1) / (FLUX_T / 32),
                     (b.n[dir] + seglen - 1) / seglen);
     if (dir == 1)
-      k_flux_pass<1, RECON, EOS, UCT><<<grid, block, 0, s>>>(a, eos, seglen);
+      launch_pass(k_flux_pass<1, RECON, EOS, UCT>, grid, block, s, a, eos, seglen);
     else
-      k_flux_pass<2, RECON, EOS, UCT><<<grid, block, 0, s>>>(a, eos, seglen);
+      launch_pass(k_flux_pass<2, RECON, EOS, UCT>, grid, block, s, a, eos, seglen);
     return cudaGetLastError() == cudaSuccess ? AXB_OK : AXB_ERR_CUDA;
   }
   // the threads walk the transverse plane [ng-1, ng+n]^2 row after row
@@ -44,11 +51,11 @@ int launch_flux_pass_uct(int dir, const RhsArgs &a, const EOS &eos, int seglen,
   RhsArgs ap = a;
   ap.b.packed = 1;
   const long long plane = (long long)(b.n[T0] + 2 * a.text) * (b.n[T1] + 2 * a.text);
-  const dim3 grid(unsigned((plane + 127) / 128), 1, (b.n[dir] + seglen - 1) / seglen);
+  const dim3 grid(unsigned((plane + FLUX_T - 1) / FLUX_T), 1, (b.n[dir] + seglen - 1) / seglen);
   if (dir == 1)
-    k_flux_pass<1, RECON, EOS, UCT><<<grid, block, 0, s>>>(ap, eos, seglen);
+    launch_pass(k_flux_pass<1, RECON, EOS, UCT>, grid, block, s, ap, eos, seglen);
   else
-    k_flux_pass<2, RECON, EOS, UCT><<<grid, block, 0, s>>>(ap, eos, seglen);
+    launch_pass(k_flux_pass<2, RECON, EOS, UCT>, grid, block, s, ap, eos, seglen);
   return cudaGetLastError() == cudaSuccess ? AXB_OK : AXB_ERR_CUDA;
 }
 
@@ -75,7 +82,7 @@ int launch_flux_pass_t(int dir, const RhsArgs &a, const axb_eos &eos,
 // Batched flux passes over the boxes of a batch (tile tables built by the
 // batch with the grids of launch_flux_pass_eos).
 template <int DIR, int RECON, class EOS>
-__global__ void __launch_bounds__(128, AXB_FLUX_MINB)
+__global__ void __launch_bounds__(FLUX_T, FLUX_MINB)
     k_flux_pass_batch(const RhsArgs *args, const TileTable t, unsigned long long *ctr, const __grid_constant__ EOS eos, const int seglen) {
   batch_loop(args, t, ctr, [&](const RhsArgs &a, const uint3 bid) {
     flux_pass_body<DIR, RECON, EOS>(a, eos, seglen, bid);
@@ -99,9 +106,11 @@ int launch_flux_batch_eos(int dir, const RhsArgs *args, const TileTable &t,
   if (dir == 0)
     k_flux_x_batch<RECON, EOS><<<nblocks, 128, 0, s>>>(args, t, ctr, eos);
   else if (dir == 1)
-    k_flux_pass_batch<1, RECON, EOS><<<nblocks, dim3(32, 4), 0, s>>>(args, t, ctr, eos, seglen);
+    launch_pass(k_flux_pass_batch<1, RECON, EOS>, dim3(nblocks), dim3(32, FLUX_T / 32), s, args,
+                t, ctr, eos, seglen);
   else
-    k_flux_pass_batch<2, RECON, EOS><<<nblocks, dim3(32, 4), 0, s>>>(args, t, ctr, eos, seglen);
+    launch_pass(k_flux_pass_batch<2, RECON, EOS>, dim3(nblocks), dim3(32, FLUX_T / 32), s, args,
+                t, ctr, eos, seglen);
   return cudaGetLastError() == cudaSuccess ? AXB_OK : AXB_ERR_CUDA;
 }
 

@@ -3,10 +3,6 @@
 
 #include "axb_rhs.cuh"
 
-#ifndef AXB_FLUX_STASH
-#define AXB_FLUX_STASH 1 // the left face state in shared memory (face_fluxes)
-#endif
-
 namespace axb {
 
 template <int N>
@@ -32,26 +28,31 @@ AXB_D double warp_max(double v) {
 // Shared pieces of the flux passes.
 // ---------------------------------------------------------------------------
 
-// Reconstruct the NREC variables of the cell at I (stride sd along DIR).
-template <int DIR, int RECON>
-AXB_D void recon_cell_all(const RhsArgs &a, const double *const (&fld)[NREC],
-                          long long I, long long sd, double (&lo)[NREC],
-                          double (&up)[NREC]) {
-  double pr[5], vd[5];
-  load_pencil<5>(a.press, I, sd, pr);
-  load_pencil<5>(a.vel[DIR], I, sd, vd);
+// Reconstruct the NREC variables of the cell at I (stride sd along DIR);
+// `win(v, m)` is variable v of the cell m - 2 cells on.  Only PPM reads the
+// pressure (its own stencil when the temperature is reconstructed) and, with
+// zone flattening, the velocity along the pencil.
+template <int DIR, int RECON, class Win>
+AXB_D void recon_cell_all(const RhsArgs &a, const Win &win, long long I, long long sd,
+                          double (&lo)[NREC], double (&up)[NREC]) {
+  double pr[5] = {}, vd[5] = {};
+  if constexpr (RECON == AXB_RECON_PPM) {
+    if (a.rec_temp) {
+      load_pencil<5>(a.press, I, sd, pr);
+    } else {
+#pragma unroll
+      for (int m = 0; m < 5; ++m)
+        pr[m] = win(R_PRESS, m);
+    }
+    if (a.rp.ppm_zone_flattening)
+      load_pencil<5>(a.vel[DIR], I, sd, vd);
+  }
 #pragma unroll
   for (int v = 0; v < NREC; ++v) {
     double q[5];
-    if (v == R_PRESS && !a.rec_temp) {
 #pragma unroll
-      for (int m = 0; m < 5; ++m) q[m] = pr[m];
-    } else if (v == R_VX + DIR && a.recvar == AXB_RECVAR_V) {
-#pragma unroll
-      for (int m = 0; m < 5; ++m) q[m] = vd[m];
-    } else {
-      load_pencil<5>(fld[v], I, sd, q);
-    }
+    for (int m = 0; m < 5; ++m)
+      q[m] = win(v, m);
     const CellLoUp r = recon_cell<RECON>(q, pr, vd, v == R_RHO, a.rp);
     lo[v] = r.lo;
     up[v] = r.up;
@@ -92,34 +93,6 @@ AXB_D void face_fluxes(const RhsArgs &a, const EOS &eos,
   const double Bdir = __ldg(a.dBstag[DIR] + I) * m.isqrtg;
   SideOut sL, sR;
   side_physics<DIR, UCT>(m, L, Bdir, eos, a.rec_temp, a.recvar, sL);
-  // (y and z passes) the left state's conserved variables and fluxes wait in
-  // shared memory while the right state is formed: held in registers, the
-  // two states together push the pencil march past its register budget
-  // (measured at 256^3: y 3.40 -> 3.21 ms, z 4.06 -> 3.79 ms; the x pass,
-  // which carries less, was not faster with it)
-  constexpr bool stash = AXB_FLUX_STASH && DIR != 0;
-  volatile double *sl = nullptr;
-  if constexpr (stash) {
-    __shared__ double s_left[20][128];
-    sl = &s_left[0][threadIdx.y * blockDim.x + threadIdx.x];
-#pragma unroll
-    for (int v = 0; v < 10; ++v) {
-      sl[128 * v] = sL.U[v];
-      sl[128 * (10 + v)] = sL.F[v];
-    }
-  }
-  auto uL = [&](int v) -> double {
-    if constexpr (stash)
-      return sl[128 * v];
-    else
-      return sL.U[v];
-  };
-  auto fL = [&](int v) -> double {
-    if constexpr (stash)
-      return sl[128 * (10 + v)];
-    else
-      return sL.F[v];
-  };
   side_physics<DIR, UCT>(m, R, Bdir, eos, a.rec_temp, a.recvar, sR);
   const double cmax = fmax(0.0, fmax(fmax(sL.lam_p, sL.lam_m), fmax(sR.lam_p, sR.lam_m)));
   const double cmin = fmin(0.0, fmin(fmin(sL.lam_p, sL.lam_m), fmin(sR.lam_p, sR.lam_m)));
@@ -128,12 +101,12 @@ AXB_D void face_fluxes(const RhsArgs &a, const EOS &eos,
     const double icpm = 1 / (cmax - cmin);
 #pragma unroll
     for (int v = 0; v < 10; ++v)
-      F[v] = hlle_flux(cmax, cmin, icpm, uL(v), sR.U[v], fL(v), sR.F[v]);
+      F[v] = hlle_flux(cmax, cmin, icpm, sL.U[v], sR.U[v], sL.F[v], sR.F[v]);
   } else {
     const double ch = fmax(cmax, -cmin);
 #pragma unroll
     for (int v = 0; v < 10; ++v)
-      F[v] = laxf_flux(ch, uL(v), sR.U[v], fL(v), sR.F[v]);
+      F[v] = laxf_flux(ch, sL.U[v], sR.U[v], sL.F[v], sR.F[v]);
   }
 #pragma unroll
   for (int v = 0; v < 10; ++v)
@@ -197,24 +170,24 @@ AXB_D void flux_status(const RhsArgs &a, double smax, bool bad, bool bad_rhs = f
              (any_bad ? AXB_EW_NAN_FLUX : 0u) | (any_rhs ? AXB_EW_NAN_RHS : 0u));
 }
 
-#ifndef AXB_FLUX_MINB
-#define AXB_FLUX_MINB 4 // resident CTAs per SM the register budget must allow
-#endif
 #ifndef AXB_FLUX_X_MINB
-#define AXB_FLUX_X_MINB 4
+#define AXB_FLUX_X_MINB 4 // resident CTAs per SM the register budget must allow
 #endif
-#ifndef AXB_FLUX_SMEM_CARRY
-#define AXB_FLUX_SMEM_CARRY 1
-#endif
-#ifndef AXB_FLUX_PREFETCH
-#define AXB_FLUX_PREFETCH 1 // steps of L2 prefetch ahead of the march (0: none)
-#endif
-#ifndef AXB_FLUX_PF_RECON
-#define AXB_FLUX_PF_RECON 1
-#endif
-#ifndef AXB_FLUX_PF_ACC
-#define AXB_FLUX_PF_ACC 1
-#endif
+constexpr int FLUX_T = 128;   // threads of a y/z pass block
+constexpr int FLUX_MINB = 3;  // its resident CTAs per SM (shared memory, registers)
+// its dynamic shared memory: ring, upper values, fluxes
+constexpr int FLUX_SMEM = (5 * NREC + NREC + NHYDRO) * FLUX_T * int(sizeof(double));
+
+// asynchronous copy of one double into shared memory, and the wait for all of
+// this thread's copies
+AXB_D void cp_async8(double *smem, const double *g) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                   unsigned(__cvta_generic_to_shared(smem))),
+               "l"(g)
+               : "memory");
+}
+AXB_D void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+AXB_D void cp_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
 // k_flux_pass (y and z): one thread marches one pencil segment along DIR.
@@ -223,6 +196,21 @@ AXB_D void flux_status(const RhsArgs &a, double smax, bool bad, bool bad_rhs = f
 // folds F(face) - F(face-1) into the partial divergence of the previous cell.
 // Threads of a warp are adjacent along x, so every load is a coalesced
 // 256-byte row.
+//
+// What bounds it is latency: 16 warps per SM re-reading their stencils through
+// the L1 that 147 KB of shared memory left them hit it 18 % of the time and
+// waited 5 (y) to 7 (z) cycles per issued instruction for L2, with the FP64
+// pipe at 36 / 31 %.  So each thread keeps its five stencil rows in shared
+// memory, a ring of five slots per variable: the next cell's last row is
+// copied asynchronously into the slot of the row just used while the face is
+// computed, and a step reads 9 doubles from memory for its stencils instead of
+// 45.  With the carried upper values and fluxes that is 488 bytes a thread;
+// three CTAs per SM fit, whose 168 registers hold both face states without
+// spills (four at 128 registers spilled, and kept the left state in shared
+// memory).  256^3 WENO-Z: y 3.55 -> 2.87 ms, z 3.80 -> 3.09 ms (beside the
+// sources).  Not kept: a four-slot ring with the last row loaded directly at
+// four CTAs (3.05 / 3.31 ms) or three (2.95 / 3.09); seven 64-thread CTAs at
+// 128 registers (3.39 / 3.66).
 // Transverse range: cells [ng-1, ng+n] (one ghost layer each side, needed
 // by the edge electric field); faces along DIR: [ng, ng+n].
 // ---------------------------------------------------------------------------
@@ -267,36 +255,32 @@ AXB_D void flux_pass_body(const RhsArgs &a, const EOS &eos, const int &seglen, c
                                      a.recv[0], a.recv[1], a.recv[2], a.Bvec[D1],
                                      a.Bvec[D2]};
     const double idxd = b.idx[DIR];
-#if AXB_FLUX_SMEM_CARRY
-    // the state carried from one cell to the next (upper interface values
-    // of the previous cell, flux of the previous face) lives in shared
-    // memory: in registers it pushed the march beyond its register budget
-    // and into local-memory spills
-    __shared__ double s_carry[NREC + NHYDRO][128];
+    extern __shared__ double s_dyn[];
     const int tl = threadIdx.y * blockDim.x + threadIdx.x;
-#define AXB_UPL(v) s_carry[v][tl]
-#define AXB_FPREV(v) s_carry[NREC + (v)][tl]
-#else
-    double upL[NREC];
-    double Fprev[NHYDRO];
-#define AXB_UPL(v) upL[v]
-#define AXB_FPREV(v) Fprev[v]
-#endif
-    for (int c = f0 - 1; c <= flast; ++c, I += sd) {
-#if AXB_FLUX_PREFETCH > 0
-      // L2 prefetch of the rows the march first touches AXB_FLUX_PREFETCH
-      // steps ahead: the new stencil row of every reconstructed variable,
-      // the face metric's two vertex rows, the face's staggered B and the
-      // partial divergences (and RHS) it will accumulate into; all of them
-      // within the rows this segment reads anyway
-      if (c + AXB_FLUX_PREFETCH <= flast) {
-        const long long J = I + AXB_FLUX_PREFETCH * sd;
-#if AXB_FLUX_PF_RECON
+    // the thread's slots: 5 rows of the stencil (a ring), the upper values of
+    // the previous cell, the fluxes of the previous face
+    double *const ring = s_dyn + tl;
+    double *const s_up = ring + 5 * NREC * FLUX_T;
+    double *const s_fprev = s_up + NREC * FLUX_T;
+    auto fetch = [&](int slot, long long J) { // a stencil row into a ring slot
 #pragma unroll
-        for (int v = 0; v < NREC; ++v)
-          prefetch_l2(fld[v] + J + 2 * sd);
-#endif
-        constexpr int D1 = (DIR + 1) % 3, D2 = (DIR + 2) % 3;
+      for (int v = 0; v < NREC; ++v)
+        cp_async8(ring + (slot + v) * FLUX_T, fld[v] + J);
+    };
+    int o[5]; // ring slots of the rows c-2 .. c+2
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
+      o[m] = m * NREC;
+      fetch(o[m], I + (m - 2) * sd);
+    }
+    cp_async_commit();
+#pragma unroll 1
+    for (int c = f0 - 1; c <= flast; ++c, I += sd) {
+      // L2 prefetch of the rows the march first touches a step ahead: the
+      // face metric's two vertex rows, the face's staggered B and the partial
+      // divergences (and RHS) it will accumulate into
+      if (c + 1 <= flast) {
+        const long long J = I + sd;
         const long long so = (D1 == 0) ? b.stride(D2) : b.stride(D1);
         prefetch_l2(a.alp + J);
         prefetch_l2(a.alp + J + so);
@@ -311,51 +295,63 @@ AXB_D void flux_pass_body(const RhsArgs &a, const EOS &eos, const int &seglen, c
           prefetch_l2(a.g[q] + J + so);
         }
         prefetch_l2(a.dBstag[DIR] + J);
-        if (AXB_FLUX_PF_ACC && trans_int) {
+        if (trans_int) {
 #pragma unroll
           for (int v = 0; v < NHYDRO; ++v) {
-            prefetch_l2(a.acc[v] + J - sd);
+            prefetch_l2(a.acc[v] + I);
             if (DIR == 2)
-              prefetch_l2(a.rhs[v] + J - sd);
+              prefetch_l2(a.rhs[v] + I);
           }
         }
       }
-#endif
+      cp_async_wait(); // this thread's own copies: no barrier
       double lo[NREC], up[NREC];
-      recon_cell_all<DIR, RECON>(a, fld, I, sd, lo, up);
+      recon_cell_all<DIR, RECON>(
+          a, [&](int v, int m) { return ring[(o[m] + v) * FLUX_T]; }, I, sd, lo, up);
+      // the next cell's last row lands in the slot of this cell's first one
+      // while the face is computed
+      if (c < flast)
+        fetch(o[0], I + 3 * sd);
+      cp_async_commit();
+      const int first = o[0];
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+        o[m] = o[m + 1];
+      o[4] = first;
       if (c >= f0) {
         // face c: left state = upper values of cell c-1, right = lower of c
-        double L[NREC], R[NREC], F[10];
+        double L[NREC], F[10];
 #pragma unroll
-        for (int v = 0; v < NREC; ++v) {
-          L[v] = AXB_UPL(v);
-          R[v] = lo[v];
-        }
-        face_fluxes<DIR, UCT>(a, eos, fld, I, sd, L, R, F, smax, bad);
+        for (int v = 0; v < NREC; ++v)
+          L[v] = s_up[v * FLUX_T];
+        // (stored ahead of the face: the face needs the registers)
+#pragma unroll
+        for (int v = 0; v < NREC; ++v)
+          s_up[v * FLUX_T] = up[v];
+        face_fluxes<DIR, UCT>(a, eos, fld, I, sd, L, lo, F, smax, bad);
         if (c > f0 && trans_int) {
           double Fc[NHYDRO], Fp[NHYDRO];
 #pragma unroll
           for (int v = 0; v < NHYDRO; ++v) {
             Fc[v] = F[v];
-            Fp[v] = AXB_FPREV(v);
+            Fp[v] = s_fprev[v * FLUX_T];
           }
           bad_rhs |= fold_divergence<DIR>(a, I - sd, idxd, Fc, Fp);
         }
 #pragma unroll
         for (int v = 0; v < NHYDRO; ++v)
-          AXB_FPREV(v) = F[v];
-      }
+          s_fprev[v * FLUX_T] = F[v];
+      } else {
 #pragma unroll
-      for (int v = 0; v < NREC; ++v)
-        AXB_UPL(v) = up[v];
+        for (int v = 0; v < NREC; ++v)
+          s_up[v * FLUX_T] = up[v];
+      }
     }
-#undef AXB_UPL
-#undef AXB_FPREV
   }
   flux_status(a, smax, bad, bad_rhs);
 }
 template <int DIR, int RECON, class EOS, bool UCT = false>
-__global__ void __launch_bounds__(128, AXB_FLUX_MINB)
+__global__ void __launch_bounds__(FLUX_T, FLUX_MINB)
     k_flux_pass(const RhsArgs a, const __grid_constant__ EOS eos, const int seglen) {
   flux_pass_body<DIR, RECON, EOS, UCT>(a, eos, seglen, blockIdx);
 }
@@ -397,7 +393,8 @@ AXB_D void flux_x_body(const RhsArgs &a, const EOS &eos, const uint3 bid) {
       const long long I = row + c;
       double lo[NREC], up[NREC];
       if (has_cell) {
-        recon_cell_all<0, RECON>(a, fld, I, 1, lo, up);
+        recon_cell_all<0, RECON>(
+            a, [&](int v, int m) { return __ldg(fld[v] + I + (m - 2)); }, I, 1, lo, up);
       } else {
 #pragma unroll
         for (int v = 0; v < NREC; ++v)
