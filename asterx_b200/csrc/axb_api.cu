@@ -1,4 +1,5 @@
 // C ABI of the engine: contexts, equations of state and the RHS group.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -648,12 +649,12 @@ int fill_rhs_args(axb_ctx *c, const axb_box *box, const axb_fields *f,
 
 namespace axb {
 int launch_flux_pass(int dir, int recon, const RhsArgs &a, const axb_eos &eos,
-                     int seglen, cudaStream_t s) {
+                     cudaStream_t s) {
   switch (recon) {
-  case AXB_RECON_PPM: return launch_flux_ppm(dir, a, eos, seglen, s);
-  case AXB_RECON_WENOZ: return launch_flux_wenoz(dir, a, eos, seglen, s);
-  case AXB_RECON_MP5: return launch_flux_mp5(dir, a, eos, seglen, s);
-  default: return launch_flux_low(recon, dir, a, eos, seglen, s);
+  case AXB_RECON_PPM: return launch_flux_ppm(dir, a, eos, s);
+  case AXB_RECON_WENOZ: return launch_flux_wenoz(dir, a, eos, s);
+  case AXB_RECON_MP5: return launch_flux_mp5(dir, a, eos, s);
+  default: return launch_flux_low(recon, dir, a, eos, s);
   }
 }
 } // namespace axb
@@ -699,10 +700,6 @@ int rhs_group_run(axb_ctx *c, const axb_box *box, const axb_fields *f,
   if (eos->kind == 1 && !a.rec_temp)
     return AXB_ERR_UNSUPPORTED;
   cudaStream_t s = (cudaStream_t)stream;
-#ifndef AXB_FLUX_SEGLEN
-#define AXB_FLUX_SEGLEN 16 // cells per y/z pencil segment (one thread each)
-#endif
-  const int seglen = AXB_FLUX_SEGLEN;
   if (!bc && side_stream(c)) {
     // the sources and the vertex auxiliaries read neither the partial
     // divergences nor the face B fluxes, and the flux passes read neither
@@ -727,7 +724,7 @@ int rhs_group_run(axb_ctx *c, const axb_box *box, const axb_fields *f,
       if (dir == 2)
         cudaStreamWaitEvent(s, c->ev_sources, 0);
       axb_mark(c, AXB_R_FLUX_X + dir, s, true);
-      rc = launch_flux_pass(dir, p->reconstruction_method, a, *eos, seglen, s);
+      rc = launch_flux_pass(dir, p->reconstruction_method, a, *eos, s);
       axb_mark(c, AXB_R_FLUX_X + dir, s, false);
     }
     // always joined back, on success or not
@@ -746,7 +743,7 @@ int rhs_group_run(axb_ctx *c, const axb_box *box, const axb_fields *f,
     return rc;
   for (int dir = 0; dir < 3; ++dir) {
     axb_mark(c, AXB_R_FLUX_X + dir, s, true);
-    rc = launch_flux_pass(dir, p->reconstruction_method, a, *eos, seglen, s);
+    rc = launch_flux_pass(dir, p->reconstruction_method, a, *eos, s);
     axb_mark(c, AXB_R_FLUX_X + dir, s, false);
     if (rc)
       return rc;
@@ -808,19 +805,25 @@ namespace axb {
 int launch_rhs_misc(int which, const RhsArgs &a, cudaStream_t s) {
   const BoxDev &b = a.b;
   const int T = 128;
-  if (which <= 1 && AXB_SOURCES_SEG > 1) {
-    const int seg = AXB_SOURCES_SEG;
-    const dim3 grid((b.n[0] + T - 1) / T, b.n[1], (b.n[2] + seg - 1) / seg);
+  if (which <= 1) {
+    // z columns of cells; the (i, j) plane row after row where rows of whole
+    // blocks would leave more of them idle
+    RhsArgs ap = a;
+    dim3 grid((b.n[0] + T - 1) / T, b.n[1], 1);
+    const long long plane = ((long long)b.n[0] * b.n[1] + T - 1) / T;
+    if (plane < (long long)grid.x * grid.y) {
+      ap.b.packed = 1;
+      grid = dim3(unsigned(plane), 1, 1);
+    }
+    const int n = b.n[2];
+    const int seg = split_steps(n, double(SOURCES_MINB) * sm_count(), SOURCES_START, [&](int q) {
+      return (long long)grid.x * grid.y * ((n + q - 1) / q);
+    });
+    grid.z = (n + seg - 1) / seg;
     if (which == 0)
-      k_sources_column<2><<<grid, T, 0, s>>>(a, seg);
+      k_sources_column<2><<<grid, T, 0, s>>>(ap, seg);
     else
-      k_sources_column<4><<<grid, T, 0, s>>>(a, seg);
-  } else if (which <= 1) {
-    const dim3 grid((b.n[0] + T - 1) / T, b.n[1], b.n[2]);
-    if (which == 0)
-      k_sources<2><<<grid, T, 0, s>>>(a);
-    else
-      k_sources<4><<<grid, T, 0, s>>>(a);
+      k_sources_column<4><<<grid, T, 0, s>>>(ap, seg);
   } else {
     // vertex and edge kernels: threads walk the (i, j) plane row after row,
     // so rows of n+5 or n+1 points do not leave a block mostly idle
@@ -856,14 +859,11 @@ int launch_rhs_misc(int which, const RhsArgs &a, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 namespace {
 template <int FD>
-__global__ void __launch_bounds__(128, AXB_SOURCES_MINB)
-    k_sources_batch(const RhsArgs *args, const TileTable t, unsigned long long *ctr) {
-  batch_loop(args, t, ctr, [&](const RhsArgs &a, const uint3 bid) {
-    if (AXB_SOURCES_SEG > 1)
-      sources_column<FD>(a, bid, AXB_SOURCES_SEG);
-    else
-      sources_body<FD>(a, bid);
-  });
+__global__ void __launch_bounds__(128, SOURCES_MINB)
+    k_sources_batch(const RhsArgs *args, const TileTable t, unsigned long long *ctr,
+                    const int seg) {
+  batch_loop(args, t, ctr,
+             [&](const RhsArgs &a, const uint3 bid) { sources_column<FD>(a, bid, seg); });
 }
 __global__ void __launch_bounds__(128) k_aux_batch(const RhsArgs *args, const TileTable t, unsigned long long *ctr) {
   batch_loop(args, t, ctr, [&](const RhsArgs &a, const uint3 bid) { aux_body(a, bid); });
@@ -874,6 +874,7 @@ __global__ void __launch_bounds__(128) k_ct_psi_batch(const RhsArgs *args, const
 } // namespace
 
 namespace axb {
+uint3 flux_grid(int dir, const axb_box &b, int seglen);
 // The per-box RHS argument blocks of a batch (checked as axb_rhs_group
 // checks them), in device memory.
 int batch_rhs_setup(axb_ctx *c, int nbox, const axb_box *boxes, const axb_fields *f,
@@ -902,31 +903,48 @@ int batch_rhs_setup(axb_ctx *c, int nbox, const axb_box *boxes, const axb_fields
   return rc;
 }
 
-// batched grids over packed (i, j) planes: 0 sources, 2 aux, 3 CT + Psi
-uint3 rhs_misc_grid(int which, const axb_box &b) {
+// batched grids over packed (i, j) planes: 0 sources (columns of `seg` cells),
+// 2 aux, 3 CT + Psi
+uint3 rhs_misc_grid(int which, const axb_box &b, int seg) {
   const int T = 128;
   const int e = which <= 1 ? 0 : which == 2 ? 5 : 1;
   const long long plane = (long long)(b.n[0] + e) * (b.n[1] + e);
-  if (which <= 1 && AXB_SOURCES_SEG > 1) // z columns of the sources
-    return make_uint3(unsigned((plane + T - 1) / T), 1,
-                      (b.n[2] + AXB_SOURCES_SEG - 1) / AXB_SOURCES_SEG);
-  return make_uint3(unsigned((plane + T - 1) / T), 1, b.n[2] + e);
+  const int nz = which <= 1 ? (b.n[2] + seg - 1) / seg : b.n[2] + e;
+  return make_uint3(unsigned((plane + T - 1) / T), 1, nz);
 }
 
 int launch_rhs_misc_batch(int which, const void *args, const TileTable &t,
-                          unsigned long long *ctr, int nblocks, cudaStream_t s) {
+                          unsigned long long *ctr, int seg, int nblocks, cudaStream_t s) {
   if (t.total == 0)
     return AXB_OK;
   const RhsArgs *a = static_cast<const RhsArgs *>(args);
   if (which == 0)
-    k_sources_batch<2><<<nblocks, 128, 0, s>>>(a, t, ctr);
+    k_sources_batch<2><<<nblocks, 128, 0, s>>>(a, t, ctr, seg);
   else if (which == 1)
-    k_sources_batch<4><<<nblocks, 128, 0, s>>>(a, t, ctr);
+    k_sources_batch<4><<<nblocks, 128, 0, s>>>(a, t, ctr, seg);
   else if (which == 2)
     k_aux_batch<<<nblocks, 128, 0, s>>>(a, t, ctr);
   else
     k_ct_psi_batch<<<nblocks, 128, 0, s>>>(a, t, ctr);
   return cudaGetLastError() == cudaSuccess ? AXB_OK : AXB_ERR_CUDA;
+}
+
+// the split of a level's marching kernels, by the tiles of all its boxes: the
+// y and z passes (dir 1, 2) or the sources' columns (dir 0)
+int batch_steps(int dir, const axb_box *boxes, int nbox, int sms) {
+  int n = 1;
+  for (int q = 0; q < nbox; ++q)
+    n = std::max(n, dir ? boxes[q].n[dir] : boxes[q].n[2]);
+  return split_steps(n, double(dir ? FLUX_MINB : SOURCES_MINB) * sms,
+                     dir ? FLUX_START : SOURCES_START, [&](int seg) {
+                       long long t = 0;
+                       for (int q = 0; q < nbox; ++q) {
+                         const uint3 g = dir ? flux_grid(dir, boxes[q], seg)
+                                             : rhs_misc_grid(0, boxes[q], seg);
+                         t += (long long)g.x * g.y * g.z;
+                       }
+                       return t;
+                     });
 }
 
 using Ctr = unsigned long long;

@@ -29,13 +29,14 @@ int batch_c2p_setup(axb_ctx *c, int nbox, const axb_box *boxes, const axb_fields
                     const axb_params *p, const axb_eos *eos, void **out);
 int batch_rk_setup(int nbox, const axb_box *boxes, const axb_fields *f, const axb_fields *fn,
                    int recvar, void **stage_args, void **sync_evolved, void **sync_prims);
-uint3 rhs_misc_grid(int which, const axb_box &b);
+uint3 rhs_misc_grid(int which, const axb_box &b, int seg);
+int batch_steps(int dir, const axb_box *boxes, int nbox, int sms);
 uint3 flux_grid(int dir, const axb_box &b, int seglen);
 uint3 stage_grid(const axb_box &b);
 uint3 sync_grid(const axb_box &b, int set);
 uint3 c2p_grid(int which, const axb_box &b);
 int launch_rhs_misc_batch(int which, const void *args, const TileTable &t,
-                          unsigned long long *ctr, int nblocks, cudaStream_t s);
+                          unsigned long long *ctr, int seg, int nblocks, cudaStream_t s);
 int launch_flux_batch(int recon, int dir, const RhsArgs *args, const TileTable &t,
                       unsigned long long *ctr, const axb_eos &eos, DevStatus *status,
                       int seglen, int nblocks, cudaStream_t s);
@@ -93,8 +94,12 @@ struct axb_batch {
   void *rhs_args = nullptr, *c2p_args = nullptr, *stage_args = nullptr;
   void *sync_e = nullptr, *sync_p = nullptr;
   DevTable tab[NPHASE];
-  DevTable flux_seg[2][NSEG]; // y, z tables per candidate segment
-  int seg[2] = {2, 2};        // index into kSeg (32)
+  // y, z tables: the autotuner's candidate segments, then the one chosen by
+  // the level's size (split_steps), which stands until the autotuner is asked
+  DevTable flux_seg[2][NSEG + 1];
+  int steps[2] = {16, 16}; // that segment
+  int seg[2] = {NSEG, NSEG}; // index of the table in use
+  int src_steps = 16;        // cells of a sources column
   int ctas[NPHASE];           // CTAs per SM of each phase's persistent grid
   unsigned long long *ctr = nullptr; // one work counter per phase
   // deferred-cell queue of the recovery's fast pass (null: full cascade)
@@ -134,18 +139,23 @@ void free_table(DevTable &d) {
   d = DevTable{};
 }
 
-uint3 g_sources(const axb_box &b, int) { return rhs_misc_grid(0, b); }
-uint3 g_aux(const axb_box &b, int) { return rhs_misc_grid(2, b); }
-uint3 g_ct(const axb_box &b, int) { return rhs_misc_grid(3, b); }
+uint3 g_sources(const axb_box &b, int seg) { return rhs_misc_grid(0, b, seg); }
+uint3 g_aux(const axb_box &b, int) { return rhs_misc_grid(2, b, 1); }
+uint3 g_ct(const axb_box &b, int) { return rhs_misc_grid(3, b, 1); }
 uint3 g_flux(const axb_box &b, int dir_seg) { return flux_grid(dir_seg & 3, b, dir_seg >> 2); }
 uint3 g_stage(const axb_box &b, int) { return stage_grid(b); }
 uint3 g_sync(const axb_box &b, int set) { return sync_grid(b, set); }
 uint3 g_c2p(const axb_box &b, int which) { return c2p_grid(which, b); }
 
-int nblocks_for(const axb_batch *B, int phase, long long total) {
-  const long long want = (total + BATCH_CHUNK - 1) / BATCH_CHUNK;
+// the persistent grid of a phase, and the items its CTAs draw at a time
+int nblocks_for(const axb_batch *B, int phase, TileTable &t) {
   const long long cap = (long long)B->ctas[phase] * B->sms;
-  return int(std::max(1LL, std::min(want, cap)));
+  t.chunk = t.total >= 16 * cap ? BATCH_CHUNK : 1;
+  return int(std::max(1LL, std::min((t.total + t.chunk - 1) / t.chunk, cap)));
+}
+
+int segment_of(const axb_batch *B, int d) {
+  return B->seg[d] < NSEG ? kSeg[B->seg[d]] : B->steps[d];
 }
 
 const TileTable &table_of(const axb_batch *B, int phase) {
@@ -158,26 +168,26 @@ const TileTable &table_of(const axb_batch *B, int phase) {
 
 int launch_phase(axb_ctx *c, const axb_batch *B, int phase, double alpha, double beta,
                  double gdt, cudaStream_t s) {
-  const TileTable &t = table_of(B, phase);
-  const int nb = nblocks_for(B, phase, t.total);
+  TileTable t = table_of(B, phase);
+  const int nb = nblocks_for(B, phase, t);
   unsigned long long *ctr = B->ctr + phase;
   axb_mark(c, kRegion[phase], s, true);
   int rc = AXB_OK;
   switch (phase) {
   case P_SOURCES:
-    rc = launch_rhs_misc_batch(B->fd_order == 4 ? 1 : 0, B->rhs_args, t, ctr, nb, s);
+    rc = launch_rhs_misc_batch(B->fd_order == 4 ? 1 : 0, B->rhs_args, t, ctr, B->src_steps, nb, s);
     break;
   case P_FLUX_X:
   case P_FLUX_Y:
   case P_FLUX_Z: {
     const int dir = phase - P_FLUX_X;
-    const int seg = dir == 0 ? 32 : kSeg[B->seg[dir - 1]];
+    const int seg = dir == 0 ? 32 : segment_of(B, dir - 1);
     rc = launch_flux_batch(B->recon, dir, static_cast<const RhsArgs *>(B->rhs_args), t, ctr,
                            *B->eos, B->status, seg, nb, s);
     break;
   }
-  case P_AUX: rc = launch_rhs_misc_batch(2, B->rhs_args, t, ctr, nb, s); break;
-  case P_CT: rc = launch_rhs_misc_batch(3, B->rhs_args, t, ctr, nb, s); break;
+  case P_AUX: rc = launch_rhs_misc_batch(2, B->rhs_args, t, ctr, 1, nb, s); break;
+  case P_CT: rc = launch_rhs_misc_batch(3, B->rhs_args, t, ctr, 1, nb, s); break;
   case P_STAGE: rc = launch_stage_batch(B->stage_args, t, ctr, alpha, beta, gdt, nb, s); break;
   case P_SYNC_E: rc = launch_sync_batch(B->sync_e, t, ctr, nb, s); break;
   case P_BSTAG: rc = launch_c2p_batch(0, B->c2p_args, t, ctr, *B->eos, B->status, nb, s); break;
@@ -250,13 +260,17 @@ AXB_API int axb_batch_create(axb_ctx *c, int nbox, const axb_box *boxes,
   if (!rc)
     rc = batch_rk_setup(nbox, boxes, fields, fields_n, p->recon_type, &B->stage_args,
                         &B->sync_e, &B->sync_p);
+  B->src_steps = batch_steps(0, boxes, nbox, B->sms);
+  for (int d = 0; d < 2; ++d)
+    B->steps[d] = batch_steps(d + 1, boxes, nbox, B->sms);
   if (!rc)
-    rc = make_table(bx, g_sources, 0, B->tab[P_SOURCES]);
+    rc = make_table(bx, g_sources, B->src_steps, B->tab[P_SOURCES]);
   if (!rc)
     rc = make_table(bx, g_flux, 0, B->tab[P_FLUX_X]);
   for (int d = 0; d < 2 && !rc; ++d)
-    for (int q = 0; q < NSEG && !rc; ++q)
-      rc = make_table(bx, g_flux, (d + 1) | (kSeg[q] << 2), B->flux_seg[d][q]);
+    for (int q = 0; q <= NSEG && !rc; ++q)
+      rc = make_table(bx, g_flux, (d + 1) | ((q < NSEG ? kSeg[q] : B->steps[d]) << 2),
+                      B->flux_seg[d][q]);
   if (!rc)
     rc = make_table(bx, g_aux, 0, B->tab[P_AUX]);
   if (!rc)
@@ -355,7 +369,7 @@ AXB_API int axb_batch_autotune(axb_ctx *c, axb_batch *B, int *out, void *stream)
   }
   // segment length of the y and z passes
   for (int d = 0; d < 2 && !rc; ++d) {
-    int best = B->seg[d];
+    int best = 0;
     float best_ms = 1e30f;
     for (int q = 0; q < NSEG && !rc; ++q) {
       B->seg[d] = q;

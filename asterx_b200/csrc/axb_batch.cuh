@@ -22,6 +22,7 @@ struct TileTable {
   const uint3 *grid;       // per-box grid of the single-box launch
   int nbox;
   long long total;
+  int chunk; // items a CTA draws at a time
 };
 
 // box of a flat item index (prefix is non-decreasing, prefix[0] = 0)
@@ -46,8 +47,9 @@ AXB_D uint3 tile_bid(const uint3 g, long long local) {
   return b;
 }
 
-// Items are handed out in chunks of this many by an atomic counter, so CTAs
-// that drew cheap tiles (small boxes) take more of them.
+// Items are handed out in chunks by an atomic counter, so CTAs that drew cheap
+// tiles (small boxes) take more of them: four at a time where every CTA of the
+// grid comes back often, else one, so that the last items spread over the GPU.
 constexpr int BATCH_CHUNK = 4;
 
 // Run f(args_of_box, block_index) over the items this CTA draws from the
@@ -65,12 +67,12 @@ AXB_D void batch_loop(const Args *__restrict__ args, const TileTable &t,
   for (;;) {
     __syncthreads();
     if (tid == 0)
-      s_base = (long long)atomicAdd(ctr, (unsigned long long)BATCH_CHUNK);
+      s_base = (long long)atomicAdd(ctr, (unsigned long long)t.chunk);
     __syncthreads();
     const long long base = s_base;
     if (base >= t.total) // CTA-uniform
       break;
-    const long long last = min(base + BATCH_CHUNK, t.total);
+    const long long last = min(base + t.chunk, t.total);
     for (long long item = base; item < last; ++item) {
       const int bx = tile_box(t, item);
       if (bx != cur) {

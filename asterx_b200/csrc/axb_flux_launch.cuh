@@ -16,8 +16,7 @@ void launch_pass(K kernel, dim3 grid, dim3 block, cudaStream_t s, const Args &..
 }
 
 template <int RECON, class EOS, bool UCT>
-int launch_flux_pass_uct(int dir, const RhsArgs &a, const EOS &eos, int seglen,
-                         cudaStream_t s) {
+int launch_flux_pass_uct(int dir, const RhsArgs &a, const EOS &eos, cudaStream_t s) {
   const BoxDev &b = a.b;
   if (dir == 0) {
     // one warp per (y, z) row of the transverse range [ng-te, ng+n+te-1]^2
@@ -28,7 +27,8 @@ int launch_flux_pass_uct(int dir, const RhsArgs &a, const EOS &eos, int seglen,
     k_flux_x<RECON, EOS, UCT><<<(unsigned)blocks, 128, 0, s>>>(a, eos);
     return cudaGetLastError() == cudaSuccess ? AXB_OK : AXB_ERR_CUDA;
   }
-  const int T0 = 0, T1 = dir == 2 ? 1 : 2;
+  const int T0 = 0, T1 = dir == 2 ? 1 : 2, n = b.n[dir];
+  const double slots = double(FLUX_MINB) * sm_count();
   const dim3 block(32, FLUX_T / 32);
   // Thread layout: 32 columns x 4 rows of the transverse plane per block,
   // or the plane walked row after row (no lane idle on the n+2-wide rows).
@@ -37,8 +37,12 @@ int launch_flux_pass_uct(int dir, const RhsArgs &a, const EOS &eos, int seglen,
   // share the face metric's second vertex row in L1).
   constexpr bool packed = RECON != AXB_RECON_MP5;
   if (!packed) {
-    const dim3 grid((b.n[T0] + 2 * a.text + 31) / 32, (b.n[T1] + 2 * a.text + FLUX_T / 32 - 1) / (FLUX_T / 32),
-                    (b.n[dir] + seglen - 1) / seglen);
+    dim3 grid((b.n[T0] + 2 * a.text + 31) / 32,
+              (b.n[T1] + 2 * a.text + FLUX_T / 32 - 1) / (FLUX_T / 32), 1);
+    const int seglen = split_steps(n, slots, FLUX_START, [&](int seg) {
+      return (long long)grid.x * grid.y * ((n + seg - 1) / seg);
+    });
+    grid.z = (n + seglen - 1) / seglen;
     if (dir == 1)
       launch_pass(k_flux_pass<1, RECON, EOS, UCT>, grid, block, s, a, eos, seglen);
     else
@@ -51,7 +55,11 @@ int launch_flux_pass_uct(int dir, const RhsArgs &a, const EOS &eos, int seglen,
   RhsArgs ap = a;
   ap.b.packed = 1;
   const long long plane = (long long)(b.n[T0] + 2 * a.text) * (b.n[T1] + 2 * a.text);
-  const dim3 grid(unsigned((plane + FLUX_T - 1) / FLUX_T), 1, (b.n[dir] + seglen - 1) / seglen);
+  dim3 grid(unsigned((plane + FLUX_T - 1) / FLUX_T), 1, 1);
+  const int seglen = split_steps(n, slots, FLUX_START, [&](int seg) {
+    return (long long)grid.x * ((n + seg - 1) / seg);
+  });
+  grid.z = (n + seglen - 1) / seglen;
   if (dir == 1)
     launch_pass(k_flux_pass<1, RECON, EOS, UCT>, grid, block, s, ap, eos, seglen);
   else
@@ -62,20 +70,18 @@ int launch_flux_pass_uct(int dir, const RhsArgs &a, const EOS &eos, int seglen,
 // the upwind-CT face data and the wider transverse range are a separate
 // instantiation, so the flux-CT passes carry none of it
 template <int RECON, class EOS>
-int launch_flux_pass_eos(int dir, const RhsArgs &a, const EOS &eos, int seglen,
-                         cudaStream_t s) {
+int launch_flux_pass_eos(int dir, const RhsArgs &a, const EOS &eos, cudaStream_t s) {
   if (a.use_uct)
-    return launch_flux_pass_uct<RECON, EOS, true>(dir, a, eos, seglen, s);
-  return launch_flux_pass_uct<RECON, EOS, false>(dir, a, eos, seglen, s);
+    return launch_flux_pass_uct<RECON, EOS, true>(dir, a, eos, s);
+  return launch_flux_pass_uct<RECON, EOS, false>(dir, a, eos, s);
 }
 
 template <int RECON>
-int launch_flux_pass_t(int dir, const RhsArgs &a, const axb_eos &eos,
-                       int seglen, cudaStream_t s) {
+int launch_flux_pass_t(int dir, const RhsArgs &a, const axb_eos &eos, cudaStream_t s) {
   if (eos.kind == 0)
-    return launch_flux_pass_eos<RECON>(dir, a, eos.ideal, seglen, s);
+    return launch_flux_pass_eos<RECON>(dir, a, eos.ideal, s);
   if (eos.kind == 1)
-    return launch_flux_pass_eos<RECON>(dir, a, tab_for_launch(eos, a.status), seglen, s);
+    return launch_flux_pass_eos<RECON>(dir, a, tab_for_launch(eos, a.status), s);
   return AXB_ERR_UNSUPPORTED;
 }
 
@@ -130,9 +136,9 @@ int launch_flux_batch(int recon, int dir, const RhsArgs *args, const TileTable &
                       unsigned long long *ctr, const axb_eos &eos, DevStatus *status,
                       int seglen, int nblocks, cudaStream_t s);
 
-int launch_flux_ppm(int dir, const RhsArgs &a, const axb_eos &eos, int seglen, cudaStream_t s);
-int launch_flux_wenoz(int dir, const RhsArgs &a, const axb_eos &eos, int seglen, cudaStream_t s);
-int launch_flux_mp5(int dir, const RhsArgs &a, const axb_eos &eos, int seglen, cudaStream_t s);
-int launch_flux_low(int recon, int dir, const RhsArgs &a, const axb_eos &eos, int seglen, cudaStream_t s);
+int launch_flux_ppm(int dir, const RhsArgs &a, const axb_eos &eos, cudaStream_t s);
+int launch_flux_wenoz(int dir, const RhsArgs &a, const axb_eos &eos, cudaStream_t s);
+int launch_flux_mp5(int dir, const RhsArgs &a, const axb_eos &eos, cudaStream_t s);
+int launch_flux_low(int recon, int dir, const RhsArgs &a, const axb_eos &eos, cudaStream_t s);
 
 } // namespace axb

@@ -1,9 +1,9 @@
 // k_flux_pass instantiations for the wenoz reconstruction.
 #include "axb_flux_launch.cuh"
 namespace axb {
-int launch_flux_wenoz(int dir, const RhsArgs &a, const axb_eos &eos, int seglen,
-                   cudaStream_t s) {
-  return launch_flux_pass_t<AXB_RECON_WENOZ>(dir, a, eos, seglen, s);
+int launch_flux_wenoz(int dir, const RhsArgs &a, const axb_eos &eos,
+                    cudaStream_t s) {
+  return launch_flux_pass_t<AXB_RECON_WENOZ>(dir, a, eos, s);
 }
 int launch_flux_batch_wenoz(int dir, const RhsArgs *args, const TileTable &t,
                           unsigned long long *ctr, const axb_eos &eos, DevStatus *st,

@@ -111,9 +111,48 @@ inline axb::EosTab tab_for_launch(const axb_eos &e, axb::DevStatus *st) {
 }
 
 namespace axb {
+// How many steps a thread of a marching kernel (a pencil of the flux passes, a
+// column of the sources) should take, for work of `blocks(seg)` blocks of
+// which `slots` are resident at once: the `seg` of the least estimated time
+//   (seg + start) x (waves of blocks),
+// `start` the steps a segment costs on top of its own (its first cell's
+// reconstruction and face).  A wave that is not full still takes a good part of
+// a full one: w = blocks / slots counts as w + half of what the last wave lacks
+// when there is more than one, and as 0.65 + 0.35 w below (fewer warps per SM
+// run faster).  Long segments repeat less work, short ones fill a GPU that a
+// small box leaves idle and even out the last wave.  Measured against the
+// fixed 16 on the y pass: 20x16x24 cells 126 us at 16, 25 at 1 (chosen); 64^3
+// 115 / 68 at 6 (chosen); 128^3 396 / 384 at 8 (chosen) / 379 at 12; 101x72x61
+// 156 / 131 at 12 (chosen); beyond 128^3 within 3 % of each other from 12 to 32.
+template <class F>
+inline int split_steps(int n, double slots, double start, const F &blocks) {
+  int best = 1;
+  double best_cost = 1e300;
+  for (int seg = 1; seg <= n && seg <= 32; ++seg) {
+    const double w = double(blocks(seg)) / slots;
+    const double up = double((long long)w + ((long long)w < w));
+    const double waves = w <= 1.0 ? 0.65 + 0.35 * w : w + 0.5 * (up - w);
+    const double cost = (seg + start) * waves;
+    if (cost <= best_cost) {
+      best_cost = cost;
+      best = seg;
+    }
+  }
+  return best;
+}
+// streaming multiprocessors of the current device
+inline int sm_count() {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess)
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+} // namespace axb
+
+namespace axb {
 // launchers (one per translation unit of kernels)
 int launch_flux_pass(int dir, int recon, const struct RhsArgs &a,
-                     const axb_eos &eos, int seglen, cudaStream_t s);
+                     const axb_eos &eos, cudaStream_t s);
 int launch_rhs_misc(int which, const struct RhsArgs &a, cudaStream_t s);
 } // namespace axb
 

@@ -277,7 +277,14 @@ int con2prim_group_run(axb_ctx *c, const axb_box *box, const axb_fields *f,
     a.bracket = mlp_device_view(mlp).bracket;
   }
   {
-    const dim3 grid((b.n[0] + T - 1) / T, b.n[1], b.n[2]);
+    // the cells of a plane row after row where rows of whole blocks would
+    // leave more of them idle
+    dim3 grid((b.n[0] + T - 1) / T, b.n[1], b.n[2]);
+    const long long plane = ((long long)b.n[0] * b.n[1] + T - 1) / T;
+    if (plane < (long long)grid.x * grid.y) {
+      a.b.packed = 1;
+      grid = dim3(unsigned(plane), 1, b.n[2]);
+    }
     axb_mark(c, AXB_R_C2P, s, true);
     const bool fast = a.c2p_prime == AXB_C2P_PALENZUELA && c2p_queue_fits(*box);
     void *buf = nullptr;

@@ -175,6 +175,7 @@ AXB_D void flux_status(const RhsArgs &a, double smax, bool bad, bool bad_rhs = f
 #endif
 constexpr int FLUX_T = 128;   // threads of a y/z pass block
 constexpr int FLUX_MINB = 3;  // its resident CTAs per SM (shared memory, registers)
+constexpr double FLUX_START = 1.2; // what starting a segment costs, in steps
 // its dynamic shared memory: ring, upper values, fluxes
 constexpr int FLUX_SMEM = (5 * NREC + NREC + NHYDRO) * FLUX_T * int(sizeof(double));
 

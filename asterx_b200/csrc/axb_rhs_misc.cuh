@@ -88,9 +88,8 @@ AXB_HD double sym_get(const sym3 &m, int p, int q) { return m(p, q); }
 #ifndef AXB_SOURCES_SMEM
 #define AXB_SOURCES_SMEM 1
 #endif
-#ifndef AXB_SOURCES_MINB
-#define AXB_SOURCES_MINB 3
-#endif
+constexpr int SOURCES_MINB = 3;       // resident CTAs per SM of the sources
+constexpr double SOURCES_START = 0.5; // what starting a column costs, in cells
 template <int FD>
 AXB_D void sources_cell(const RhsArgs &a, const int i, const int j, const int k) {
   const BoxDev &b = a.b;
@@ -237,22 +236,10 @@ AXB_D void sources_cell(const RhsArgs &a, const int i, const int j, const int k)
   a.rhs[V_TAU][I] = as * tau_source;
   a.rhs[V_DYE][I] = 0.0;
 }
-template <int FD>
-AXB_D void sources_body(const RhsArgs &a, const uint3 bid) {
-  int i, j;
-  const int k = a.b.ng + bid.z;
-  if (!a.b.row_ij(a.b.ng, a.b.n[0], a.b.ng, a.b.n[1], bid, i, j))
-    return;
-  sources_cell<FD>(a, i, j, k);
-}
-
 // A thread walks `seg` cells up a z column (block z = segment), prefetching
 // into L2 the rows the next cell adds: the upper vertex plane of the 16
 // metric fields and the cell's primitives (its lower vertex plane is the
 // current cell's upper one).
-#ifndef AXB_SOURCES_SEG
-#define AXB_SOURCES_SEG 16 // cells per thread along z; 0 or 1: one cell
-#endif
 template <int FD>
 AXB_D void sources_column(const RhsArgs &a, const uint3 bid, const int seg) {
   const BoxDev &b = a.b;
@@ -294,12 +281,7 @@ AXB_D void sources_column(const RhsArgs &a, const uint3 bid, const int seg) {
 }
 
 template <int FD>
-__global__ void __launch_bounds__(128, AXB_SOURCES_MINB)
-    k_sources(const RhsArgs a) {
-  sources_body<FD>(a, blockIdx);
-}
-template <int FD>
-__global__ void __launch_bounds__(128, AXB_SOURCES_MINB)
+__global__ void __launch_bounds__(128, SOURCES_MINB)
     k_sources_column(const RhsArgs a, const int seg) {
   sources_column<FD>(a, blockIdx, seg);
 }
