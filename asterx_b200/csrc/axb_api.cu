@@ -973,12 +973,11 @@ int launch_flux_batch(int recon, int dir, const RhsArgs *args, const TileTable &
 }
 
 // batched grid of a flux pass: the x pass as launch_flux_pass_eos (a 1-D
-// grid of 4-warp blocks over the rows), the y and z passes over the packed
+// grid of 4-warp blocks over the rows end to end), the y and z passes over the packed
 // transverse plane (128 pencils per block) times the segments along dir
 uint3 flux_grid(int dir, const axb_box &b, int seglen) {
   if (dir == 0) {
-    const long long warps = (long long)(b.n[1] + 2) * (b.n[2] + 2);
-    return make_uint3(unsigned((warps * 32 + 127) / 128), 1, 1);
+    return make_uint3(unsigned(flux_x_blocks(make_box(b), 1)), 1, 1);
   }
   const int T1 = dir == 2 ? 1 : 2;
   const long long plane = (long long)(b.n[0] + 2) * (b.n[T1] + 2);

@@ -19,9 +19,7 @@ template <int RECON, class EOS, bool UCT>
 int launch_flux_pass_uct(int dir, const RhsArgs &a, const EOS &eos, cudaStream_t s) {
   const BoxDev &b = a.b;
   if (dir == 0) {
-    // one warp per (y, z) row of the transverse range [ng-te, ng+n+te-1]^2
-    const long long warps = (long long)(b.n[1] + 2 * a.text) * (b.n[2] + 2 * a.text);
-    const long long blocks = (warps * 32 + 127) / 128;
+    const long long blocks = flux_x_blocks(b, a.text);
     if (blocks > 0x7fffffffLL)
       return AXB_ERR_TOO_LARGE;
     k_flux_x<RECON, EOS, UCT><<<(unsigned)blocks, 128, 0, s>>>(a, eos);
