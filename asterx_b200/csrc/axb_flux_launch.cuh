@@ -27,29 +27,12 @@ int launch_flux_pass_uct(int dir, const RhsArgs &a, const EOS &eos, cudaStream_t
   }
   const int T0 = 0, T1 = dir == 2 ? 1 : 2, n = b.n[dir];
   const double slots = double(FLUX_MINB) * sm_count();
-  const dim3 block(32, FLUX_T / 32);
-  // Thread layout: 32 columns x 4 rows of the transverse plane per block,
-  // or the plane walked row after row (no lane idle on the n+2-wide rows).
-  // Measured at 256^3: the packed walk is 7-9 % faster for WENO-Z and PPM,
-  // while MP5 is 30 % faster on the 32 x 4 blocks (each block's four rows
-  // share the face metric's second vertex row in L1).
-  constexpr bool packed = RECON != AXB_RECON_MP5;
-  if (!packed) {
-    dim3 grid((b.n[T0] + 2 * a.text + 31) / 32,
-              (b.n[T1] + 2 * a.text + FLUX_T / 32 - 1) / (FLUX_T / 32), 1);
-    const int seglen = split_steps(n, slots, FLUX_START, [&](int seg) {
-      return (long long)grid.x * grid.y * ((n + seg - 1) / seg);
-    });
-    grid.z = (n + seglen - 1) / seglen;
-    if (dir == 1)
-      launch_pass(k_flux_pass<1, RECON, EOS, UCT>, grid, block, s, a, eos, seglen);
-    else
-      launch_pass(k_flux_pass<2, RECON, EOS, UCT>, grid, block, s, a, eos, seglen);
-    return cudaGetLastError() == cudaSuccess ? AXB_OK : AXB_ERR_CUDA;
-  }
-  // the threads walk the transverse plane [ng-1, ng+n]^2 row after row
-  // (as in the batched kernels), so the 2 extra columns of the plane do
-  // not leave most of a warp idle
+  const dim3 block(FLUX_T);
+  // The threads walk the transverse plane [ng-1, ng+n]^2 row after row (as in
+  // the batched kernels), so the 2 extra columns of the plane do not leave most
+  // of a warp idle.  (Blocks of 32 columns x 4 rows, which MP5 was faster on
+  // while its stencils came through L1: 128^3 substep 3.19 ms, 2.88 so; 96^3
+  // tabulated RHS 3.49 ms, 2.48 so.)
   RhsArgs ap = a;
   ap.b.packed = 1;
   const long long plane = (long long)(b.n[T0] + 2 * a.text) * (b.n[T1] + 2 * a.text);
@@ -110,10 +93,10 @@ int launch_flux_batch_eos(int dir, const RhsArgs *args, const TileTable &t,
   if (dir == 0)
     k_flux_x_batch<RECON, EOS><<<nblocks, 128, 0, s>>>(args, t, ctr, eos);
   else if (dir == 1)
-    launch_pass(k_flux_pass_batch<1, RECON, EOS>, dim3(nblocks), dim3(32, FLUX_T / 32), s, args,
+    launch_pass(k_flux_pass_batch<1, RECON, EOS>, dim3(nblocks), dim3(FLUX_T), s, args,
                 t, ctr, eos, seglen);
   else
-    launch_pass(k_flux_pass_batch<2, RECON, EOS>, dim3(nblocks), dim3(32, FLUX_T / 32), s, args,
+    launch_pass(k_flux_pass_batch<2, RECON, EOS>, dim3(nblocks), dim3(FLUX_T), s, args,
                 t, ctr, eos, seglen);
   return cudaGetLastError() == cudaSuccess ? AXB_OK : AXB_ERR_CUDA;
 }

@@ -162,7 +162,7 @@ AXB_D void flux_status(const RhsArgs &a, double smax, bool bad, bool bad_rhs = f
   // raises it (all of them on one address would serialise; a stale read only
   // costs an atomic too many)
   smax = warp_max(smax);
-  const bool lead = (threadIdx.x + threadIdx.y * blockDim.x) % 32 == 0;
+  const bool lead = threadIdx.x % 32 == 0;
   if (lead && smax > __longlong_as_double(*(volatile long long *)&a.status->max_speed_bits))
     atomic_max_nonneg(&a.status->max_speed_bits, smax);
   const bool any_bad = __any_sync(0xffffffffu, bad);
@@ -226,21 +226,12 @@ AXB_D void flux_pass_body(const RhsArgs &a, const EOS &eos, const int &seglen, c
   const BoxDev &b = a.b;
   const int ng = b.ng;
   constexpr int te = UCT ? 3 : 1; // transverse ghost layers covered
-  int t0, t1;
-  bool active;
-  if (b.packed) {
-    // (batched small boxes) the block's threads walk the transverse plane
-    // [ng-te, ng+n+te-1]^2 row after row, so short rows leave no lane idle
-    const int w0 = b.n[T0] + 2 * te;
-    const int flat = bid.x * (blockDim.x * blockDim.y) + threadIdx.y * blockDim.x + threadIdx.x;
-    t0 = ng - te + flat % w0;
-    t1 = ng - te + flat / w0;
-    active = flat < w0 * (b.n[T1] + 2 * te);
-  } else {
-    t0 = ng - te + bid.x * blockDim.x + threadIdx.x;
-    t1 = ng - te + bid.y * blockDim.y + threadIdx.y;
-    active = (t0 <= ng + b.n[T0] + te - 1) && (t1 <= ng + b.n[T1] + te - 1);
-  }
+  // the block's threads walk the transverse plane [ng-te, ng+n+te-1]^2 row
+  // after row
+  const int w0 = b.n[T0] + 2 * te;
+  const int flat = bid.x * FLUX_T + threadIdx.x;
+  const int t0 = ng - te + flat % w0, t1 = ng - te + flat / w0;
+  const bool active = flat < w0 * (b.n[T1] + 2 * te);
   double smax = 0.0;
   bool bad = false, bad_rhs = false;
   if (active) {
@@ -259,10 +250,9 @@ AXB_D void flux_pass_body(const RhsArgs &a, const EOS &eos, const int &seglen, c
                                      a.Bvec[D2]};
     const double idxd = b.idx[DIR];
     extern __shared__ double s_dyn[];
-    const int tl = threadIdx.y * blockDim.x + threadIdx.x;
     // the thread's slots: 5 rows of the stencil (a ring), the upper values of
     // the previous cell, the fluxes of the previous face
-    double *const ring = s_dyn + tl;
+    double *const ring = s_dyn + threadIdx.x;
     double *const s_up = ring + 5 * NREC * FLUX_T;
     double *const s_fprev = s_up + NREC * FLUX_T;
     auto fetch = [&](int slot, long long J) { // a stencil row into a ring slot
