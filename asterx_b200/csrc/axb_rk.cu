@@ -60,26 +60,39 @@ __global__ void __launch_bounds__(128)
   rk_stage_body(a, a.alpha, a.beta, a.gdt, blockIdx);
 }
 
-struct SyncArgs {
+// The fields of a ghost fill, those of one centring together: group q holds
+// f[first[q] .. first[q + 1]).  Eight centrings at most; NF bounds the fields.
+template <int NF> struct SyncArgsN {
   BoxDev b;
-  double *f[AXB_NUM_GF];
-  int cent[AXB_NUM_GF][3];
-  int nf;
+  double *f[NF];
+  int first[9];
+  int cent[8][3];
+  int groups;
+  int small; // ghost points fit 32 bits
 };
+using SyncArgs = SyncArgsN<AXB_NUM_GF>;
+using SyncArgsBatch = SyncArgsN<16>; // a substep's fields (11 or up to 15)
 
+// the periodic image of i; a ghost layer is no wider than the box (n >= ng),
+// and a vertex-centred direction has one point more
 AXB_D int wrap(int i, int ng, int n) {
-  int r = (i - ng) % n;
+  int r = i - ng;
   if (r < 0)
     r += n;
-  return ng + r;
+  else if (r >= n)
+    r -= n;
+  return ng + (r < n ? r : r - n);
 }
 
 // Periodic ghost fill: every point outside the interior of its centring
 // takes the value of its periodic image inside the interior.  One thread per
 // ghost point, enumerated slab below, slab above, then the ghost rows and
 // row ends of the middle planes, so no thread idles on interior points.
-struct Shell {
-  long long A, B, Cm, G;
+// Ghost points are counted in 32 bits where they fit (Int = unsigned): the
+// enumeration is four divisions per point, and 64-bit ones took most of the
+// kernel's time.
+template <class Int> struct Shell {
+  Int plane, A, AB, Cm, G;
   int N[3], hi[3], ng;
   AXB_HD Shell(const BoxDev &b, const int c[3]) {
     ng = b.ng;
@@ -87,57 +100,86 @@ struct Shell {
       N[d] = b.n[d] + 2 * ng + (c[d] ? 0 : 1);
       hi[d] = ng + b.n[d] + (c[d] ? 0 : 1);
     }
-    const long long plane = (long long)N[0] * N[1];
-    A = ng * plane;
-    B = (long long)(N[2] - hi[2]) * plane;
-    Cm = (long long)(ng + N[1] - hi[1]) * N[0] + (long long)(hi[1] - ng) * (ng + N[0] - hi[0]);
-    G = A + B + (long long)(hi[2] - ng) * Cm;
+    plane = Int(N[0]) * Int(N[1]);
+    A = Int(ng) * plane;
+    AB = A + Int(N[2] - hi[2]) * plane;
+    Cm = Int(ng + N[1] - hi[1]) * Int(N[0]) + Int(hi[1] - ng) * Int(ng + N[0] - hi[0]);
+    G = AB + Int(hi[2] - ng) * Cm;
   }
-  AXB_HD void point(long long g, int &i, int &j, int &k) const {
-    const long long plane = (long long)N[0] * N[1];
-    if (g < A + B) {
-      k = g < A ? int(g / plane) : hi[2] + int((g - A) / plane);
-      const long long r = g < A ? g % plane : (g - A) % plane;
-      j = int(r / N[0]);
-      i = int(r % N[0]);
+  AXB_HD void point(Int g, int &i, int &j, int &k) const {
+    if (g < AB) {
+      const Int q = g < A ? g : g - A;
+      const Int z = q / plane, r = q - z * plane;
+      k = (g < A ? 0 : hi[2]) + int(z);
+      j = int(r / Int(N[0]));
+      i = int(r - Int(j) * Int(N[0]));
       return;
     }
-    g -= A + B;
-    k = ng + int(g / Cm);
-    long long r = g % Cm;
-    const long long lowrows = (long long)ng * N[0], highrows = (long long)(N[1] - hi[1]) * N[0];
-    if (r < lowrows) {
-      j = int(r / N[0]);
-      i = int(r % N[0]);
-    } else if (r < lowrows + highrows) {
-      r -= lowrows;
-      j = hi[1] + int(r / N[0]);
-      i = int(r % N[0]);
+    g -= AB;
+    const Int z = g / Cm;
+    Int r = g - z * Cm;
+    k = ng + int(z);
+    const Int lowrows = Int(ng) * Int(N[0]), rows = lowrows + Int(N[1] - hi[1]) * Int(N[0]);
+    if (r < rows) {
+      j = int(r / Int(N[0]));
+      i = int(r - Int(j) * Int(N[0]));
+      if (r >= lowrows)
+        j += hi[1] - ng;
     } else {
-      r -= lowrows + highrows;
-      const int per = ng + N[0] - hi[0];
-      j = ng + int(r / per);
-      const int q = int(r % per);
+      r -= rows;
+      const Int per = Int(ng + N[0] - hi[0]);
+      const Int y = r / per;
+      const int q = int(r - y * per);
+      j = ng + int(y);
       i = q < ng ? q : hi[0] + (q - ng);
     }
   }
 };
 
-AXB_D void sync_shell_body(const SyncArgs &a, const uint3 bid) {
+// One ghost point of every field of a group: its place and its image are found
+// once (a launch with a thread per field's point spent its time on them: 256^3,
+// two fills 255 -> 218 us with 32-bit divisions -> 205 us in groups; a level
+// of 64 boxes 718 -> 618 -> 304 us, where a tile's block of arguments cost
+// more than its 128 points).
+template <class Int, class Args>
+AXB_D void sync_shell_point(const Args &a, const int group, const long long g) {
   const BoxDev &b = a.b;
-  const int v = bid.z;
-  const Shell sh(b, a.cent[v]);
-  const long long g = (long long)bid.x * blockDim.x + threadIdx.x;
-  if (g >= sh.G)
+  const Shell<Int> sh(b, a.cent[group]);
+  if (g >= (long long)sh.G)
     return;
   int i, j, k;
-  sh.point(g, i, j, k);
+  sh.point(Int(g), i, j, k);
   const int ng = b.ng;
   const int is = (i >= ng && i < sh.hi[0]) ? i : wrap(i, ng, b.n[0]);
   const int js = (j >= ng && j < sh.hi[1]) ? j : wrap(j, ng, b.n[1]);
   const int ks = (k >= ng && k < sh.hi[2]) ? k : wrap(k, ng, b.n[2]);
-  double *f = a.f[v];
-  f[b.at(i, j, k)] = f[b.at(is, js, ks)];
+  const long long to = b.at(i, j, k), from = b.at(is, js, ks);
+  const int last = a.first[group + 1];
+  for (int q = a.first[group]; q < last; q += 4) {
+    double v[4]; // four loads in flight
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (q + u < last)
+        v[u] = a.f[q + u][from];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (q + u < last)
+        a.f[q + u][to] = v[u];
+  }
+}
+template <class Args> AXB_D void sync_shell_body(const Args &a, const uint3 bid) {
+  const long long g = (long long)bid.x * blockDim.x + threadIdx.x;
+  if (a.small)
+    sync_shell_point<unsigned>(a, bid.z, g);
+  else
+    sync_shell_point<long long>(a, bid.z, g);
+}
+// whether a box's points can be counted in 32 bits
+bool sync_small(const BoxDev &b) {
+  double pts = 1;
+  for (int d = 0; d < 3; ++d)
+    pts *= b.n[d] + 2.0 * b.ng + 1;
+  return pts < 2147483648.0;
 }
 
 __global__ void __launch_bounds__(128) k_sync_shell(const SyncArgs a) {
@@ -165,6 +207,31 @@ int centring_of(int gf, int c[3]) {
       c[0] = c[1] = c[2] = 0;
   }
   return 0;
+}
+
+// sorts the fields ids[0..n) of `f` into groups of one centring; false when
+// one is missing
+template <class Args>
+bool sync_groups(Args &a, const axb_fields *f, const int *ids, int n) {
+  a.groups = 0;
+  int at = 0;
+  for (int code = 0; code < 8; ++code) {
+    const int before = at;
+    for (int q = 0; q < n; ++q) {
+      int c[3];
+      centring_of(ids[q], c);
+      if (c[0] + 2 * c[1] + 4 * c[2] != code)
+        continue;
+      if (!(a.f[at++] = f->gf[ids[q]]))
+        return false;
+      for (int d = 0; d < 3; ++d)
+        a.cent[a.groups][d] = c[d];
+    }
+    if (at > before)
+      a.first[a.groups++] = before;
+  }
+  a.first[a.groups] = at;
+  return true;
 }
 
 } // namespace
@@ -220,18 +287,17 @@ AXB_API int axb_sync_periodic(axb_ctx *c, const axb_box *box,
       return AXB_ERR_ARG; // a ghost layer must fit inside one period
   SyncArgs a;
   a.b = make_box(*box);
-  a.nf = nids;
-  for (int q = 0; q < nids; ++q) {
-    if (ids[q] < 0 || ids[q] >= AXB_NUM_GF || !f->gf[ids[q]])
+  a.small = sync_small(a.b);
+  for (int q = 0; q < nids; ++q)
+    if (ids[q] < 0 || ids[q] >= AXB_NUM_GF)
       return AXB_ERR_ARG;
-    a.f[q] = f->gf[ids[q]];
-    centring_of(ids[q], a.cent[q]);
-  }
+  if (!sync_groups(a, f, ids, nids))
+    return AXB_ERR_ARG;
   // one thread per ghost point of the largest centring among the fields
   long long gmax = 0;
-  for (int q = 0; q < nids; ++q)
-    gmax = std::max(gmax, Shell(a.b, a.cent[q]).G);
-  const dim3 grid(unsigned((gmax + 127) / 128), 1, nids);
+  for (int q = 0; q < a.groups; ++q)
+    gmax = std::max(gmax, Shell<long long>(a.b, a.cent[q]).G);
+  const dim3 grid(unsigned((gmax + 127) / 128), 1, a.groups);
   axb_mark(c, AXB_R_SYNC, (cudaStream_t)stream, true);
   k_sync_shell<<<grid, 128, 0, (cudaStream_t)stream>>>(a);
   axb_mark(c, AXB_R_SYNC, (cudaStream_t)stream, false);
@@ -252,8 +318,9 @@ __global__ void __launch_bounds__(128)
 }
 
 __global__ void __launch_bounds__(128)
-    k_sync_batch(const SyncArgs *args, const TileTable t, unsigned long long *ctr) {
-  batch_loop(args, t, ctr, [&](const SyncArgs &a, const uint3 bid) { sync_shell_body(a, bid); });
+    k_sync_batch(const SyncArgsBatch *args, const TileTable t, unsigned long long *ctr) {
+  batch_loop(args, t, ctr,
+             [&](const SyncArgsBatch &a, const uint3 bid) { sync_shell_body(a, bid); });
 }
 
 template <class T> int upload(const std::vector<T> &h, void **out) {
@@ -287,7 +354,7 @@ int batch_rk_setup(int nbox, const axb_box *boxes, const axb_fields *f, const ax
       prims[nprims++] = first + q;
   }
   std::vector<StageArgs> st(nbox);
-  std::vector<SyncArgs> se(nbox), sp(nbox);
+  std::vector<SyncArgsBatch> se(nbox), sp(nbox);
   for (int b = 0; b < nbox; ++b) {
     const axb_box &box = boxes[b];
     if (box.ng < 1)
@@ -310,18 +377,12 @@ int batch_rk_setup(int nbox, const axb_box *boxes, const axb_fields *f, const ax
         a.cent[v][d] = kCent[v][d];
     }
     for (int pass = 0; pass < 2; ++pass) {
-      SyncArgs &y = pass ? sp[b] : se[b];
+      SyncArgsBatch &y = pass ? sp[b] : se[b];
       std::memset(&y, 0, sizeof y);
       y.b = make_box(box);
-      const int nf = pass ? nprims : NEVOLVED;
-      y.nf = nf;
-      for (int q = 0; q < nf; ++q) {
-        const int id = pass ? prims[q] : kEvolved[q];
-        y.f[q] = f[b].gf[id];
-        if (!y.f[q])
-          return AXB_ERR_ARG;
-        centring_of(id, y.cent[q]);
-      }
+      y.small = sync_small(y.b);
+      if (!sync_groups(y, f + b, pass ? prims : kEvolved, pass ? nprims : NEVOLVED))
+        return AXB_ERR_ARG;
     }
   }
   int rc = upload(st, stage_args);
@@ -339,21 +400,16 @@ uint3 stage_grid(const axb_box &b) {
   const long long plane = (long long)(b.n[0] + 1) * (b.n[1] + 1);
   return make_uint3(unsigned((plane + 127) / 128), 1, b.n[2] + 1);
 }
-// set 0: the 11 evolved variables; 1: the 12 cell-centred primitives; 2: the
-// primitives and the reconstructed zvec or svec (15 cell-centred fields)
+// set 0: the evolved variables (cells, three edges, vertices); else the
+// primitives (cells)
 uint3 sync_grid(const axb_box &b, int set) {
   const BoxDev bd = make_box(b);
+  const int cents[5][3] = {{1, 1, 1}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {0, 0, 0}};
+  const int groups = set == 0 ? 5 : 1;
   long long g = 0;
-  const int nf = set == 0 ? NEVOLVED : set == 1 ? 12 : 15;
-  for (int q = 0; q < nf; ++q) {
-    int c[3] = {1, 1, 1};
-    if (!set)
-      for (int d = 0; d < 3; ++d)
-        c[d] = kCent[q][d];
-    const Shell sh(bd, c);
-    g = std::max(g, sh.G);
-  }
-  return make_uint3(unsigned((g + 127) / 128), 1, nf);
+  for (int q = 0; q < groups; ++q)
+    g = std::max(g, Shell<long long>(bd, cents[q]).G);
+  return make_uint3(unsigned((g + 127) / 128), 1, groups);
 }
 
 int launch_stage_batch(const void *args, const TileTable &t, unsigned long long *ctr,
@@ -369,7 +425,7 @@ int launch_sync_batch(const void *args, const TileTable &t, unsigned long long *
                       int nblocks, cudaStream_t s) {
   if (t.total == 0)
     return AXB_OK;
-  k_sync_batch<<<nblocks, 128, 0, s>>>(static_cast<const SyncArgs *>(args), t, ctr);
+  k_sync_batch<<<nblocks, 128, 0, s>>>(static_cast<const SyncArgsBatch *>(args), t, ctr);
   return cudaGetLastError() == cudaSuccess ? AXB_OK : AXB_ERR_CUDA;
 }
 
