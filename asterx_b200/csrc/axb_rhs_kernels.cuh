@@ -137,18 +137,32 @@ template <int DIR>
 AXB_D bool fold_divergence(const RhsArgs &a, long long I, double idxd,
                            const double (&Fhi)[NHYDRO], const double (&Flo)[NHYDRO]) {
   bool bad = false;
+  // every load ahead of the first store: the arrays may not be told apart, and
+  // one at a time each variable waited for memory on its own
+  double acc[NHYDRO], rhs[NHYDRO], un[NHYDRO], uk[NHYDRO];
+#pragma unroll
+  for (int v = 0; v < NHYDRO; ++v) {
+    if (DIR != 0)
+      acc[v] = a.acc[v][I];
+    if (DIR == 2) {
+      rhs[v] = a.rhs[v][I];
+      if (a.fuse_stage) {
+        un[v] = a.st_un[v][I];
+        uk[v] = a.st_uk[v][I];
+      }
+    }
+  }
 #pragma unroll
   for (int v = 0; v < NHYDRO; ++v) {
     const double dF = Fhi[v] - Flo[v];
     if (DIR == 0) {
       a.acc[v][I] = idxd * dF;
     } else if (DIR == 1) {
-      a.acc[v][I] = a.acc[v][I] + idxd * dF;
+      a.acc[v][I] = acc[v] + idxd * dF;
     } else {
-      const double r = a.rhs[v][I] + (-(a.acc[v][I] + idxd * dF));
+      const double r = rhs[v] + (-(acc[v] + idxd * dF));
       if (a.fuse_stage)
-        a.st_uk[v][I] = stage_combine(a.st_alpha, a.st_un[v][I], a.st_beta,
-                                      a.st_uk[v][I], a.st_gdt, r);
+        a.st_uk[v][I] = stage_combine(a.st_alpha, un[v], a.st_beta, uk[v], a.st_gdt, r);
       else
         a.rhs[v][I] = r;
       bad |= !isfinite(r);

@@ -385,9 +385,15 @@ AXB_D void ct_psi_body(const RhsArgs &a, const uint3 bid) {
   const int ijk[3] = {i, j, k};
   const bool gl = a.gauge == AXB_GAUGE_GEN_LORENZ;
   const double *G = a.aux[6];
+  // the four results first, then the stores: the arrays may not be told apart,
+  // and a store between them would hold back the next one's loads
+  double r[4] = {0.0, 0.0, 0.0, 0.0}, un[4], uk[4];
+  bool in[4];
   // bflux: 0 fxBy 1 fxBz 2 fyBx 3 fyBz 4 fzBx 5 fzBy
+#pragma unroll
   for (int e = 0; e < 3; ++e) {
-    if (ijk[e] >= ng + b.n[e])
+    in[e] = ijk[e] < ng + b.n[e];
+    if (!in[e])
       continue;
     double E;
     if constexpr (UCT_RECON >= 0) {
@@ -408,17 +414,14 @@ AXB_D void ct_psi_body(const RhsArgs &a, const uint3 bid) {
       }
       E = 0.25 * ((fjk[I] + fjk[I - b.stride(ej)]) - (fkj[I] + fkj[I - b.stride(ek)]));
     }
-    double r = -E;
+    r[e] = -E;
     if (gl)
-      r = -E - (G[I + b.stride(e)] - G[I]) / b.dx[e];
-    if (a.fuse_stage)
-      a.st_uk[7 + e][I] = stage_combine(a.st_alpha, a.st_un[7 + e][I], a.st_beta,
-                                        a.st_uk[7 + e][I], a.st_gdt, r);
-    else
-      a.Arhs[e][I] = r;
+      r[e] = -E - (G[I + b.stride(e)] - G[I]) / b.dx[e];
   }
+  in[3] = true;
   if (gl) {
     double dF = 0.0;
+#pragma unroll
     for (int d = 0; d < 3; ++d) {
       const long long s = b.stride(d);
       const double *F = a.aux[d], *Fb = a.aux[3 + d];
@@ -429,19 +432,27 @@ AXB_D void ct_psi_body(const RhsArgs &a, const uint3 bid) {
           (0.5 / b.dx[d]);
       dF += c2c - one;
     }
-    const double r = -dF - a.lorenz_damp_fac * a.alp[I] * a.Psi[I];
-    if (a.fuse_stage) // Psi is read above at this vertex only
-      a.st_uk[10][I] = stage_combine(a.st_alpha, a.st_un[10][I], a.st_beta,
-                                     a.st_uk[10][I], a.st_gdt, r);
-    else
-      a.Psi_rhs[I] = r;
-  } else {
-    if (a.fuse_stage)
-      a.st_uk[10][I] = stage_combine(a.st_alpha, a.st_un[10][I], a.st_beta,
-                                     a.st_uk[10][I], a.st_gdt, 0.0);
-    else
-      a.Psi_rhs[I] = 0.0;
+    r[3] = -dF - a.lorenz_damp_fac * a.alp[I] * a.Psi[I];
   }
+  if (a.fuse_stage) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (in[e]) {
+        un[e] = a.st_un[7 + e][I];
+        uk[e] = a.st_uk[7 + e][I]; // (Psi is read above at this vertex only)
+      }
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    if (in[e]) {
+      if (a.fuse_stage)
+        a.st_uk[7 + e][I] =
+            stage_combine(a.st_alpha, un[e], a.st_beta, uk[e], a.st_gdt, r[e]);
+      else if (e < 3)
+        a.Arhs[e][I] = r[e];
+      else
+        a.Psi_rhs[I] = r[e];
+    }
 }
 __global__ void __launch_bounds__(128)
     k_ct_psi(const RhsArgs a) {
