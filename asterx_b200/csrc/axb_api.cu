@@ -660,6 +660,22 @@ int launch_flux_pass(int dir, int recon, const RhsArgs &a, const axb_eos &eos,
 } // namespace axb
 
 namespace {
+// the evolved fields a fused stage update reads and writes; false when one is
+// missing
+bool stage_fields(const axb_fields &f, const axb_fields &un, RhsArgs &a) {
+  static const int evolved[11] = {AXB_GF_dens,   AXB_GF_momx,   AXB_GF_momy,
+                                  AXB_GF_momz,   AXB_GF_tau,    AXB_GF_DYe,
+                                  AXB_GF_DEnt,   AXB_GF_Avec_x, AXB_GF_Avec_y,
+                                  AXB_GF_Avec_z, AXB_GF_Psi};
+  for (int v = 0; v < 11; ++v) {
+    a.st_un[v] = un.gf[evolved[v]];
+    a.st_uk[v] = f.gf[evolved[v]];
+    if (!a.st_un[v] || !a.st_uk[v])
+      return false;
+  }
+  return true;
+}
+
 // The stage update a substep fuses into its RHS group.
 struct StageFuse {
   const axb_fields *un;
@@ -677,18 +693,8 @@ int rhs_group_run(axb_ctx *c, const axb_box *box, const axb_fields *f,
     return rc;
   a.fuse_stage = 0;
   if (fuse) {
-    static const int evolved[11] = {AXB_GF_dens,   AXB_GF_momx,   AXB_GF_momy,
-                                    AXB_GF_momz,   AXB_GF_tau,    AXB_GF_DYe,
-                                    AXB_GF_DEnt,   AXB_GF_Avec_x, AXB_GF_Avec_y,
-                                    AXB_GF_Avec_z, AXB_GF_Psi};
-    if (!fuse->un)
+    if (!fuse->un || !stage_fields(*f, *fuse->un, a))
       return AXB_ERR_ARG;
-    for (int v = 0; v < 11; ++v) {
-      a.st_un[v] = fuse->un->gf[evolved[v]];
-      a.st_uk[v] = f->gf[evolved[v]];
-      if (!a.st_un[v] || !a.st_uk[v])
-        return AXB_ERR_ARG;
-    }
     a.fuse_stage = 1;
     a.st_alpha = fuse->alpha;
     a.st_beta = fuse->beta;
@@ -868,8 +874,11 @@ __global__ void __launch_bounds__(128, SOURCES_MINB)
 __global__ void __launch_bounds__(128) k_aux_batch(const RhsArgs *args, const TileTable t, unsigned long long *ctr) {
   batch_loop(args, t, ctr, [&](const RhsArgs &a, const uint3 bid) { aux_body(a, bid); });
 }
-__global__ void __launch_bounds__(128) k_ct_psi_batch(const RhsArgs *args, const TileTable t, unsigned long long *ctr) {
-  batch_loop(args, t, ctr, [&](const RhsArgs &a, const uint3 bid) { ct_psi_body<-1>(a, bid); });
+__global__ void __launch_bounds__(128)
+    k_ct_psi_batch(const RhsArgs *args, const TileTable t, unsigned long long *ctr,
+                   const BatchStage stage) {
+  batch_loop(
+      args, t, ctr, [&](const RhsArgs &a, const uint3 bid) { ct_psi_body<-1>(a, bid); }, stage);
 }
 } // namespace
 
@@ -878,7 +887,7 @@ uint3 flux_grid(int dir, const axb_box &b, int seglen);
 // The per-box RHS argument blocks of a batch (checked as axb_rhs_group
 // checks them), in device memory.
 int batch_rhs_setup(axb_ctx *c, int nbox, const axb_box *boxes, const axb_fields *f,
-                    const axb_params *p, const axb_eos *eos, void **out) {
+                    const axb_fields *fn, const axb_params *p, const axb_eos *eos, void **out) {
   *out = nullptr;
   RhsArgs *h = new (std::nothrow) RhsArgs[nbox];
   if (!h)
@@ -888,6 +897,8 @@ int batch_rhs_setup(axb_ctx *c, int nbox, const axb_box *boxes, const axb_fields
     if (!rc && p->use_uct)
       rc = AXB_ERR_UNSUPPORTED; // the batched CT kernel is flux CT only
     h[b].b.packed = 1;
+    if (!rc && !stage_fields(f[b], fn[b], h[b]))
+      rc = AXB_ERR_ARG;
     if (!rc && eos->kind == 1 && !h[b].rec_temp)
       rc = AXB_ERR_UNSUPPORTED;
     if (rc) {
@@ -914,7 +925,8 @@ uint3 rhs_misc_grid(int which, const axb_box &b, int seg) {
 }
 
 int launch_rhs_misc_batch(int which, const void *args, const TileTable &t,
-                          unsigned long long *ctr, int seg, int nblocks, cudaStream_t s) {
+                          unsigned long long *ctr, int seg, const BatchStage &stage, int nblocks,
+                          cudaStream_t s) {
   if (t.total == 0)
     return AXB_OK;
   const RhsArgs *a = static_cast<const RhsArgs *>(args);
@@ -925,7 +937,7 @@ int launch_rhs_misc_batch(int which, const void *args, const TileTable &t,
   else if (which == 2)
     k_aux_batch<<<nblocks, 128, 0, s>>>(a, t, ctr);
   else
-    k_ct_psi_batch<<<nblocks, 128, 0, s>>>(a, t, ctr);
+    k_ct_psi_batch<<<nblocks, 128, 0, s>>>(a, t, ctr, stage);
   return cudaGetLastError() == cudaSuccess ? AXB_OK : AXB_ERR_CUDA;
 }
 
@@ -949,26 +961,27 @@ int batch_steps(int dir, const axb_box *boxes, int nbox, int sms) {
 
 using Ctr = unsigned long long;
 int launch_flux_batch_ppm(int, const RhsArgs *, const TileTable &, Ctr *, const axb_eos &,
-                          DevStatus *, int, int, cudaStream_t);
+                          DevStatus *, int, const BatchStage &, int, cudaStream_t);
 int launch_flux_batch_wenoz(int, const RhsArgs *, const TileTable &, Ctr *, const axb_eos &,
-                            DevStatus *, int, int, cudaStream_t);
+                            DevStatus *, int, const BatchStage &, int, cudaStream_t);
 int launch_flux_batch_mp5(int, const RhsArgs *, const TileTable &, Ctr *, const axb_eos &,
-                          DevStatus *, int, int, cudaStream_t);
+                          DevStatus *, int, const BatchStage &, int, cudaStream_t);
 int launch_flux_batch_low(int, int, const RhsArgs *, const TileTable &, Ctr *,
-                          const axb_eos &, DevStatus *, int, int, cudaStream_t);
+                          const axb_eos &, DevStatus *, int, const BatchStage &, int,
+                          cudaStream_t);
 
 int launch_flux_batch(int recon, int dir, const RhsArgs *args, const TileTable &t, Ctr *ctr,
-                      const axb_eos &eos, DevStatus *st, int seglen, int nblocks,
-                      cudaStream_t s) {
+                      const axb_eos &eos, DevStatus *st, int seglen, const BatchStage &stage,
+                      int nblocks, cudaStream_t s) {
   switch (recon) {
   case AXB_RECON_PPM:
-    return launch_flux_batch_ppm(dir, args, t, ctr, eos, st, seglen, nblocks, s);
+    return launch_flux_batch_ppm(dir, args, t, ctr, eos, st, seglen, stage, nblocks, s);
   case AXB_RECON_WENOZ:
-    return launch_flux_batch_wenoz(dir, args, t, ctr, eos, st, seglen, nblocks, s);
+    return launch_flux_batch_wenoz(dir, args, t, ctr, eos, st, seglen, stage, nblocks, s);
   case AXB_RECON_MP5:
-    return launch_flux_batch_mp5(dir, args, t, ctr, eos, st, seglen, nblocks, s);
+    return launch_flux_batch_mp5(dir, args, t, ctr, eos, st, seglen, stage, nblocks, s);
   default:
-    return launch_flux_batch_low(recon, dir, args, t, ctr, eos, st, seglen, nblocks, s);
+    return launch_flux_batch_low(recon, dir, args, t, ctr, eos, st, seglen, stage, nblocks, s);
   }
 }
 

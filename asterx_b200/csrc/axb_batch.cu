@@ -5,7 +5,7 @@
 // every level), so a level of 512 small boxes costs ~5600 kernel launches per
 // substep.  Here every phase of the substep is ONE persistent launch over the
 // tiles of all boxes (axb_batch.cuh), the per-box argument blocks live in
-// device memory, and the whole substep (12 launches plus one memset of the
+// device memory, and the whole substep (11 launches plus one memset of the
 // work counters) is stream-ordered and allocation-free, so a caller can
 // capture it in a CUDA graph.  The autotuner picks the pencil segment length
 // of the y and z flux passes and the number of resident CTAs per SM of the
@@ -24,24 +24,22 @@ using namespace axb;
 namespace axb {
 // from the kernel translation units
 int batch_rhs_setup(axb_ctx *c, int nbox, const axb_box *boxes, const axb_fields *f,
-                    const axb_params *p, const axb_eos *eos, void **out);
+                    const axb_fields *fn, const axb_params *p, const axb_eos *eos, void **out);
 int batch_c2p_setup(axb_ctx *c, int nbox, const axb_box *boxes, const axb_fields *f,
                     const axb_params *p, const axb_eos *eos, void **out);
-int batch_rk_setup(int nbox, const axb_box *boxes, const axb_fields *f, const axb_fields *fn,
-                   int recvar, void **stage_args, void **sync_evolved, void **sync_prims);
+int batch_sync_setup(int nbox, const axb_box *boxes, const axb_fields *f, int recvar,
+                     void **sync_evolved, void **sync_prims);
 uint3 rhs_misc_grid(int which, const axb_box &b, int seg);
 int batch_steps(int dir, const axb_box *boxes, int nbox, int sms);
 uint3 flux_grid(int dir, const axb_box &b, int seglen);
-uint3 stage_grid(const axb_box &b);
 uint3 sync_grid(const axb_box &b, int set);
 uint3 c2p_grid(int which, const axb_box &b);
 int launch_rhs_misc_batch(int which, const void *args, const TileTable &t,
-                          unsigned long long *ctr, int seg, int nblocks, cudaStream_t s);
+                          unsigned long long *ctr, int seg, const BatchStage &stage, int nblocks,
+                          cudaStream_t s);
 int launch_flux_batch(int recon, int dir, const RhsArgs *args, const TileTable &t,
                       unsigned long long *ctr, const axb_eos &eos, DevStatus *status,
-                      int seglen, int nblocks, cudaStream_t s);
-int launch_stage_batch(const void *args, const TileTable &t, unsigned long long *ctr,
-                       double alpha, double beta, double gdt, int nblocks, cudaStream_t s);
+                      int seglen, const BatchStage &stage, int nblocks, cudaStream_t s);
 int launch_sync_batch(const void *args, const TileTable &t, unsigned long long *ctr,
                       int nblocks, cudaStream_t s);
 int launch_c2p_batch(int which, const void *args, const TileTable &t,
@@ -60,7 +58,6 @@ enum Phase {
   P_FLUX_Z,
   P_AUX,
   P_CT,
-  P_STAGE,
   P_SYNC_E,
   P_BSTAG,
   P_C2P,
@@ -68,7 +65,7 @@ enum Phase {
   NPHASE
 };
 const int kRegion[NPHASE] = {AXB_R_SOURCES, AXB_R_FLUX_X, AXB_R_FLUX_Y, AXB_R_FLUX_Z,
-                             AXB_R_AUX,     AXB_R_CT,     AXB_R_STAGE,  AXB_R_SYNC,
+                             AXB_R_AUX,     AXB_R_CT,     AXB_R_SYNC,
                              AXB_R_BSTAG,   AXB_R_C2P,    AXB_R_SYNC};
 // candidate pencil segments of the y / z flux passes
 const int kSeg[] = {8, 16, 32, 64};
@@ -91,7 +88,7 @@ struct axb_batch {
   int recon = 0, fd_order = 2;
   const axb_eos *eos = nullptr;
   DevStatus *status = nullptr;
-  void *rhs_args = nullptr, *c2p_args = nullptr, *stage_args = nullptr;
+  void *rhs_args = nullptr, *c2p_args = nullptr;
   void *sync_e = nullptr, *sync_p = nullptr;
   DevTable tab[NPHASE];
   // y, z tables: the autotuner's candidate segments, then the one chosen by
@@ -143,7 +140,6 @@ uint3 g_sources(const axb_box &b, int seg) { return rhs_misc_grid(0, b, seg); }
 uint3 g_aux(const axb_box &b, int) { return rhs_misc_grid(2, b, 1); }
 uint3 g_ct(const axb_box &b, int) { return rhs_misc_grid(3, b, 1); }
 uint3 g_flux(const axb_box &b, int dir_seg) { return flux_grid(dir_seg & 3, b, dir_seg >> 2); }
-uint3 g_stage(const axb_box &b, int) { return stage_grid(b); }
 uint3 g_sync(const axb_box &b, int set) { return sync_grid(b, set); }
 uint3 g_c2p(const axb_box &b, int which) { return c2p_grid(which, b); }
 
@@ -166,8 +162,10 @@ const TileTable &table_of(const axb_batch *B, int phase) {
   return B->tab[phase].t;
 }
 
-int launch_phase(axb_ctx *c, const axb_batch *B, int phase, double alpha, double beta,
-                 double gdt, cudaStream_t s) {
+// one phase; `stage`: the update the z pass and the CT kernel make (or the RHS
+// they store)
+int launch_phase(axb_ctx *c, const axb_batch *B, int phase, const BatchStage &stage,
+                 cudaStream_t s) {
   TileTable t = table_of(B, phase);
   const int nb = nblocks_for(B, phase, t);
   unsigned long long *ctr = B->ctr + phase;
@@ -175,7 +173,7 @@ int launch_phase(axb_ctx *c, const axb_batch *B, int phase, double alpha, double
   int rc = AXB_OK;
   switch (phase) {
   case P_SOURCES:
-    rc = launch_rhs_misc_batch(B->fd_order == 4 ? 1 : 0, B->rhs_args, t, ctr, B->src_steps, nb, s);
+    rc = launch_rhs_misc_batch(B->fd_order == 4 ? 1 : 0, B->rhs_args, t, ctr, B->src_steps, stage, nb, s);
     break;
   case P_FLUX_X:
   case P_FLUX_Y:
@@ -183,12 +181,11 @@ int launch_phase(axb_ctx *c, const axb_batch *B, int phase, double alpha, double
     const int dir = phase - P_FLUX_X;
     const int seg = dir == 0 ? 32 : segment_of(B, dir - 1);
     rc = launch_flux_batch(B->recon, dir, static_cast<const RhsArgs *>(B->rhs_args), t, ctr,
-                           *B->eos, B->status, seg, nb, s);
+                           *B->eos, B->status, seg, stage, nb, s);
     break;
   }
-  case P_AUX: rc = launch_rhs_misc_batch(2, B->rhs_args, t, ctr, 1, nb, s); break;
-  case P_CT: rc = launch_rhs_misc_batch(3, B->rhs_args, t, ctr, 1, nb, s); break;
-  case P_STAGE: rc = launch_stage_batch(B->stage_args, t, ctr, alpha, beta, gdt, nb, s); break;
+  case P_AUX: rc = launch_rhs_misc_batch(2, B->rhs_args, t, ctr, 1, stage, nb, s); break;
+  case P_CT: rc = launch_rhs_misc_batch(3, B->rhs_args, t, ctr, 1, stage, nb, s); break;
   case P_SYNC_E: rc = launch_sync_batch(B->sync_e, t, ctr, nb, s); break;
   case P_BSTAG: rc = launch_c2p_batch(0, B->c2p_args, t, ctr, *B->eos, B->status, nb, s); break;
   case P_C2P:
@@ -203,7 +200,7 @@ int launch_phase(axb_ctx *c, const axb_batch *B, int phase, double alpha, double
 
 int run_rhs_phases(axb_ctx *c, const axb_batch *B, cudaStream_t s) {
   for (int ph = P_SOURCES; ph <= P_CT; ++ph) {
-    const int rc = launch_phase(c, B, ph, 0, 0, 0, s);
+    const int rc = launch_phase(c, B, ph, BatchStage{}, s);
     if (rc)
       return rc;
   }
@@ -220,7 +217,6 @@ AXB_API int axb_batch_destroy(axb_batch *B) {
     return AXB_ERR_ARG;
   cudaFree(B->rhs_args);
   cudaFree(B->c2p_args);
-  cudaFree(B->stage_args);
   cudaFree(B->sync_e);
   cudaFree(B->sync_p);
   cudaFree(B->ctr);
@@ -254,12 +250,11 @@ AXB_API int axb_batch_create(axb_ctx *c, int nbox, const axb_box *boxes,
   std::vector<axb_box> bx(boxes, boxes + nbox);
   for (const auto &b : bx)
     B->zones += (long long)b.n[0] * b.n[1] * b.n[2];
-  int rc = batch_rhs_setup(c, nbox, boxes, fields, p, eos, &B->rhs_args);
+  int rc = batch_rhs_setup(c, nbox, boxes, fields, fields_n, p, eos, &B->rhs_args);
   if (!rc)
     rc = batch_c2p_setup(c, nbox, boxes, fields, p, eos, &B->c2p_args);
   if (!rc)
-    rc = batch_rk_setup(nbox, boxes, fields, fields_n, p->recon_type, &B->stage_args,
-                        &B->sync_e, &B->sync_p);
+    rc = batch_sync_setup(nbox, boxes, fields, p->recon_type, &B->sync_e, &B->sync_p);
   B->src_steps = batch_steps(0, boxes, nbox, B->sms);
   for (int d = 0; d < 2; ++d)
     B->steps[d] = batch_steps(d + 1, boxes, nbox, B->sms);
@@ -275,8 +270,6 @@ AXB_API int axb_batch_create(axb_ctx *c, int nbox, const axb_box *boxes,
     rc = make_table(bx, g_aux, 0, B->tab[P_AUX]);
   if (!rc)
     rc = make_table(bx, g_ct, 0, B->tab[P_CT]);
-  if (!rc)
-    rc = make_table(bx, g_stage, 0, B->tab[P_STAGE]);
   if (!rc)
     rc = make_table(bx, g_sync, 0, B->tab[P_SYNC_E]);
   if (!rc)
@@ -301,18 +294,19 @@ AXB_API int axb_batch_create(axb_ctx *c, int nbox, const axb_box *boxes,
 }
 
 // One RK substep of every box of the batch (as axb_substep does for one box):
-// RHS group, stage update, periodic fill of the evolved variables, post-step
-// group, periodic fill of the primitives.
+// RHS group with the stage update in its last kernels, periodic fill of the
+// evolved variables, post-step group, periodic fill of the primitives.
 AXB_API int axb_batch_substep(axb_ctx *c, axb_batch *B, double alpha, double beta,
                               double gamma, double dt, int periodic, void *stream) {
   if (!c || !B)
     return AXB_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   AXB_CUDA_TRY(cudaMemsetAsync(B->ctr, 0, NPHASE * sizeof(unsigned long long), s));
+  const BatchStage stage{1, alpha, beta, gamma * dt};
   for (int ph = 0; ph < NPHASE; ++ph) {
     if (!periodic && (ph == P_SYNC_E || ph == P_SYNC_P))
       continue;
-    const int rc = launch_phase(c, B, ph, alpha, beta, gamma * dt, s);
+    const int rc = launch_phase(c, B, ph, stage, s);
     if (rc)
       return rc;
   }
@@ -341,7 +335,7 @@ AXB_API int axb_batch_autotune(axb_ctx *c, axb_batch *B, int *out, void *stream)
     for (int ph = P_SOURCES; ph <= P_CT; ++ph) {
       if (ph == phase)
         AXB_CUDA_TRY(cudaEventRecord(e0, s));
-      const int rc = launch_phase(c, B, ph, 0, 0, 0, s);
+      const int rc = launch_phase(c, B, ph, BatchStage{}, s);
       if (rc)
         return rc;
       if (ph == phase)
@@ -382,8 +376,8 @@ AXB_API int axb_batch_autotune(axb_ctx *c, axb_batch *B, int *out, void *stream)
     }
     B->seg[d] = best;
   }
-  // the post-step and stage phases take the flux passes' grid size
-  B->ctas[P_STAGE] = B->ctas[P_SYNC_E] = B->ctas[P_SYNC_P] = B->ctas[P_AUX];
+  // the post-step phases take the flux passes' grid size
+  B->ctas[P_SYNC_E] = B->ctas[P_SYNC_P] = B->ctas[P_AUX];
   B->ctas[P_BSTAG] = B->ctas[P_AUX];
   B->ctas[P_C2P] = B->ctas[P_FLUX_Y];
   if (!rc)

@@ -54,10 +54,15 @@ constexpr int BATCH_CHUNK = 4;
 
 // Run f(args_of_box, block_index) over the items this CTA draws from the
 // work counter `ctr` (zeroed before the launch).  The loop ends when the
-// counter passes the item count; it never waits on other CTAs.
-template <class Args, class F>
+// counter passes the item count; it never waits on other CTAs.  `set(args)`
+// completes a box's block in shared memory with what changes from call to call
+// (one thread runs it).
+struct BatchAsIs {
+  template <class Args> AXB_D void operator()(Args &) const {}
+};
+template <class Args, class F, class Set = BatchAsIs>
 AXB_D void batch_loop(const Args *__restrict__ args, const TileTable &t,
-                      unsigned long long *ctr, F &&f) {
+                      unsigned long long *ctr, F &&f, const Set &set = Set{}) {
   __shared__ __align__(16) unsigned char raw[sizeof(Args)];
   __shared__ long long s_base;
   Args &a = *reinterpret_cast<Args *>(raw);
@@ -82,6 +87,11 @@ AXB_D void batch_loop(const Args *__restrict__ args, const TileTable &t,
         for (int q = tid; q < int(sizeof(Args) / 4); q += nthreads)
           dst[q] = __ldg(src + q);
         __syncthreads();
+        if constexpr (!std::is_same_v<Set, BatchAsIs>) {
+          if (tid == 0)
+            set(a);
+          __syncthreads();
+        }
         cur = bx;
       }
       const uint3 bid = tile_bid(t.grid[bx], item - __ldg(t.prefix + bx));

@@ -70,10 +70,14 @@ int launch_flux_pass_t(int dir, const RhsArgs &a, const axb_eos &eos, cudaStream
 // batch with the grids of launch_flux_pass_eos).
 template <int DIR, int RECON, class EOS>
 __global__ void __launch_bounds__(FLUX_T, FLUX_MINB)
-    k_flux_pass_batch(const RhsArgs *args, const TileTable t, unsigned long long *ctr, const __grid_constant__ EOS eos, const int seglen) {
-  batch_loop(args, t, ctr, [&](const RhsArgs &a, const uint3 bid) {
-    flux_pass_body<DIR, RECON, EOS>(a, eos, seglen, bid);
-  });
+    k_flux_pass_batch(const RhsArgs *args, const TileTable t, unsigned long long *ctr,
+                      const __grid_constant__ EOS eos, const int seglen, const BatchStage stage) {
+  batch_loop(
+      args, t, ctr,
+      [&](const RhsArgs &a, const uint3 bid) {
+        flux_pass_body<DIR, RECON, EOS>(a, eos, seglen, bid);
+      },
+      stage);
 }
 
 template <int RECON, class EOS>
@@ -86,36 +90,37 @@ __global__ void __launch_bounds__(128, AXB_FLUX_X_MINB)
 
 template <int RECON, class EOS>
 int launch_flux_batch_eos(int dir, const RhsArgs *args, const TileTable &t,
-                          unsigned long long *ctr, const EOS &eos, int seglen, int nblocks,
-                          cudaStream_t s) {
+                          unsigned long long *ctr, const EOS &eos, int seglen,
+                          const BatchStage &stage, int nblocks, cudaStream_t s) {
   if (t.total == 0)
     return AXB_OK;
   if (dir == 0)
     k_flux_x_batch<RECON, EOS><<<nblocks, 128, 0, s>>>(args, t, ctr, eos);
   else if (dir == 1)
     launch_pass(k_flux_pass_batch<1, RECON, EOS>, dim3(nblocks), dim3(FLUX_T), s, args,
-                t, ctr, eos, seglen);
+                t, ctr, eos, seglen, stage);
   else
     launch_pass(k_flux_pass_batch<2, RECON, EOS>, dim3(nblocks), dim3(FLUX_T), s, args,
-                t, ctr, eos, seglen);
+                t, ctr, eos, seglen, stage);
   return cudaGetLastError() == cudaSuccess ? AXB_OK : AXB_ERR_CUDA;
 }
 
 template <int RECON>
 int launch_flux_batch_t(int dir, const RhsArgs *args, const TileTable &t,
                         unsigned long long *ctr, const axb_eos &eos, DevStatus *status,
-                        int seglen, int nblocks, cudaStream_t s) {
+                        int seglen, const BatchStage &stage, int nblocks, cudaStream_t s) {
   if (eos.kind == 0)
-    return launch_flux_batch_eos<RECON>(dir, args, t, ctr, eos.ideal, seglen, nblocks, s);
+    return launch_flux_batch_eos<RECON>(dir, args, t, ctr, eos.ideal, seglen, stage, nblocks,
+                                        s);
   if (eos.kind == 1)
     return launch_flux_batch_eos<RECON>(dir, args, t, ctr, tab_for_launch(eos, status), seglen,
-                                        nblocks, s);
+                                        stage, nblocks, s);
   return AXB_ERR_UNSUPPORTED;
 }
 
 int launch_flux_batch(int recon, int dir, const RhsArgs *args, const TileTable &t,
                       unsigned long long *ctr, const axb_eos &eos, DevStatus *status,
-                      int seglen, int nblocks, cudaStream_t s);
+                      int seglen, const BatchStage &stage, int nblocks, cudaStream_t s);
 
 int launch_flux_ppm(int dir, const RhsArgs &a, const axb_eos &eos, cudaStream_t s);
 int launch_flux_wenoz(int dir, const RhsArgs &a, const axb_eos &eos, cudaStream_t s);

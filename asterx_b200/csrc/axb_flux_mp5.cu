@@ -7,7 +7,9 @@ int launch_flux_mp5(int dir, const RhsArgs &a, const axb_eos &eos,
 }
 int launch_flux_batch_mp5(int dir, const RhsArgs *args, const TileTable &t,
                           unsigned long long *ctr, const axb_eos &eos, DevStatus *st,
-                          int seglen, int nblocks, cudaStream_t s) {
-  return launch_flux_batch_t<AXB_RECON_MP5>(dir, args, t, ctr, eos, st, seglen, nblocks, s);
+                          int seglen, const BatchStage &stage, int nblocks,
+                          cudaStream_t s) {
+  return launch_flux_batch_t<AXB_RECON_MP5>(dir, args, t, ctr, eos, st, seglen, stage,
+                                                  nblocks, s);
 }
 } // namespace axb

@@ -65,6 +65,19 @@ struct RhsArgs {
   DevStatus *status;
 };
 
+// A level's stage update fused into its z pass and CT kernel (their argument
+// blocks stay on the device from call to call, the coefficients do not).
+struct BatchStage {
+  int fuse;
+  double alpha, beta, gdt;
+  AXB_D void operator()(RhsArgs &a) const {
+    a.fuse_stage = fuse;
+    a.st_alpha = alpha;
+    a.st_beta = beta;
+    a.st_gdt = gdt;
+  }
+};
+
 // Fast magnetosonic speeds of one face state (eigenvalues.hxx:19-79): the
 // roots of a2 l^2 + a1 l + a0 = 0 divided by the lapse, lam_p with +sqrt
 // and lam_m with -sqrt (the reference lists each twice).  One reciprocal of

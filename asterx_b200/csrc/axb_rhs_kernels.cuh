@@ -139,34 +139,32 @@ AXB_D bool fold_divergence(const RhsArgs &a, long long I, double idxd,
   bool bad = false;
   // every load ahead of the first store: the arrays may not be told apart, and
   // one at a time each variable waited for memory on its own
-  double acc[NHYDRO], rhs[NHYDRO], un[NHYDRO], uk[NHYDRO];
-#pragma unroll
-  for (int v = 0; v < NHYDRO; ++v) {
-    if (DIR != 0)
-      acc[v] = a.acc[v][I];
-    if (DIR == 2) {
-      rhs[v] = a.rhs[v][I];
-      if (a.fuse_stage) {
-        un[v] = a.st_un[v][I];
-        uk[v] = a.st_uk[v][I];
-      }
-    }
-  }
+  double r[NHYDRO], un[NHYDRO], uk[NHYDRO];
 #pragma unroll
   for (int v = 0; v < NHYDRO; ++v) {
     const double dF = Fhi[v] - Flo[v];
     if (DIR == 0) {
-      a.acc[v][I] = idxd * dF;
+      r[v] = idxd * dF;
     } else if (DIR == 1) {
-      a.acc[v][I] = acc[v] + idxd * dF;
+      r[v] = a.acc[v][I] + idxd * dF;
     } else {
-      const double r = rhs[v] + (-(acc[v] + idxd * dF));
-      if (a.fuse_stage)
-        a.st_uk[v][I] = stage_combine(a.st_alpha, un[v], a.st_beta, uk[v], a.st_gdt, r);
-      else
-        a.rhs[v][I] = r;
-      bad |= !isfinite(r);
+      r[v] = a.rhs[v][I] + (-(a.acc[v][I] + idxd * dF));
+      bad |= !isfinite(r[v]);
     }
+  }
+  if (DIR == 2 && a.fuse_stage) {
+#pragma unroll
+    for (int v = 0; v < NHYDRO; ++v) {
+      un[v] = a.st_un[v][I];
+      uk[v] = a.st_uk[v][I];
+    }
+#pragma unroll
+    for (int v = 0; v < NHYDRO; ++v)
+      a.st_uk[v][I] = stage_combine(a.st_alpha, un[v], a.st_beta, uk[v], a.st_gdt, r[v]);
+  } else {
+#pragma unroll
+    for (int v = 0; v < NHYDRO; ++v)
+      (DIR == 2 ? a.rhs : a.acc)[v][I] = r[v];
   }
   return bad;
 }
@@ -306,8 +304,13 @@ AXB_D void flux_pass_body(const RhsArgs &a, const EOS &eos, const int &seglen, c
 #pragma unroll
           for (int v = 0; v < NHYDRO; ++v) {
             prefetch_l2(a.acc[v] + I);
-            if (DIR == 2)
+            if (DIR == 2) {
               prefetch_l2(a.rhs[v] + I);
+              if (a.fuse_stage) {
+                prefetch_l2(a.st_un[v] + I);
+                prefetch_l2(a.st_uk[v] + I);
+              }
+            }
           }
         }
       }

@@ -310,14 +310,6 @@ AXB_API int axb_sync_periodic(axb_ctx *c, const axb_box *box,
 namespace {
 
 __global__ void __launch_bounds__(128)
-    k_rk_stage_batch(const StageArgs *args, const TileTable t, unsigned long long *ctr, double alpha, double beta,
-                     double gdt) {
-  batch_loop(args, t, ctr, [&](const StageArgs &a, const uint3 bid) {
-    rk_stage_body(a, alpha, beta, gdt, bid);
-  });
-}
-
-__global__ void __launch_bounds__(128)
     k_sync_batch(const SyncArgsBatch *args, const TileTable t, unsigned long long *ctr) {
   batch_loop(args, t, ctr,
              [&](const SyncArgsBatch &a, const uint3 bid) { sync_shell_body(a, bid); });
@@ -339,9 +331,9 @@ template <class T> int upload(const std::vector<T> &h, void **out) {
 
 namespace axb {
 
-// Per-box stage and ghost-fill argument blocks of a batch, in device memory.
-int batch_rk_setup(int nbox, const axb_box *boxes, const axb_fields *f, const axb_fields *fn,
-                   int recvar, void **stage_args, void **sync_evolved, void **sync_prims) {
+// Per-box ghost-fill argument blocks of a batch, in device memory.
+int batch_sync_setup(int nbox, const axb_box *boxes, const axb_fields *f, int recvar,
+                     void **sync_evolved, void **sync_prims) {
   // the 12 cell-centred primitives, plus the reconstructed zvec or svec
   // when the fluxes reconstruct one of those instead of the velocity
   int prims[15] = {AXB_GF_rho,   AXB_GF_velx, AXB_GF_vely,        AXB_GF_velz,
@@ -353,7 +345,6 @@ int batch_rk_setup(int nbox, const axb_box *boxes, const axb_fields *f, const ax
     for (int q = 0; q < 3; ++q)
       prims[nprims++] = first + q;
   }
-  std::vector<StageArgs> st(nbox);
   std::vector<SyncArgsBatch> se(nbox), sp(nbox);
   for (int b = 0; b < nbox; ++b) {
     const axb_box &box = boxes[b];
@@ -362,20 +353,6 @@ int batch_rk_setup(int nbox, const axb_box *boxes, const axb_fields *f, const ax
     for (int d = 0; d < 3; ++d)
       if (box.n[d] < box.ng)
         return AXB_ERR_ARG;
-    StageArgs &a = st[b];
-    std::memset(&a, 0, sizeof a);
-    a.b = make_box(box);
-    a.b.packed = 1;
-    for (int v = 0; v < NEVOLVED; ++v) {
-      a.out[v] = f[b].gf[kEvolved[v]];
-      a.un[v] = fn[b].gf[kEvolved[v]];
-      a.uk[v] = f[b].gf[kEvolved[v]];
-      a.rhs[v] = f[b].gf[kEvolvedRhs[v]];
-      if (!a.out[v] || !a.un[v] || !a.rhs[v])
-        return AXB_ERR_ARG;
-      for (int d = 0; d < 3; ++d)
-        a.cent[v][d] = kCent[v][d];
-    }
     for (int pass = 0; pass < 2; ++pass) {
       SyncArgsBatch &y = pass ? sp[b] : se[b];
       std::memset(&y, 0, sizeof y);
@@ -385,21 +362,13 @@ int batch_rk_setup(int nbox, const axb_box *boxes, const axb_fields *f, const ax
         return AXB_ERR_ARG;
     }
   }
-  int rc = upload(st, stage_args);
-  if (!rc)
-    rc = upload(se, sync_evolved);
+  int rc = upload(se, sync_evolved);
   if (!rc)
     rc = upload(sp, sync_prims);
   return rc;
 }
 
-// batched grids: the stage update over packed (i, j) planes, and the ghost
-// fill over the ghost points of the largest centring of the set (0: the 11
-// evolved variables, 1: the 12 cell-centred primitives)
-uint3 stage_grid(const axb_box &b) {
-  const long long plane = (long long)(b.n[0] + 1) * (b.n[1] + 1);
-  return make_uint3(unsigned((plane + 127) / 128), 1, b.n[2] + 1);
-}
+// batched grid of a ghost fill over the ghost points of the largest centring;
 // set 0: the evolved variables (cells, three edges, vertices); else the
 // primitives (cells)
 uint3 sync_grid(const axb_box &b, int set) {
@@ -410,15 +379,6 @@ uint3 sync_grid(const axb_box &b, int set) {
   for (int q = 0; q < groups; ++q)
     g = std::max(g, Shell<long long>(bd, cents[q]).G);
   return make_uint3(unsigned((g + 127) / 128), 1, groups);
-}
-
-int launch_stage_batch(const void *args, const TileTable &t, unsigned long long *ctr,
-                       double alpha, double beta, double gdt, int nblocks, cudaStream_t s) {
-  if (t.total == 0)
-    return AXB_OK;
-  k_rk_stage_batch<<<nblocks, 128, 0, s>>>(static_cast<const StageArgs *>(args), t, ctr,
-                                           alpha, beta, gdt);
-  return cudaGetLastError() == cudaSuccess ? AXB_OK : AXB_ERR_CUDA;
 }
 
 int launch_sync_batch(const void *args, const TileTable &t, unsigned long long *ctr,

@@ -450,7 +450,7 @@ AXB_API int axb_batch_create(axb_ctx *ctx, int nbox, const axb_box *boxes,
                              axb_batch **out);
 AXB_API int axb_batch_destroy(axb_batch *batch);
 
-/* One RK substep of every box (axb_substep semantics), as 12 stream-ordered
+/* One RK substep of every box (axb_substep semantics), as 11 stream-ordered
  * launches and one memset, allocation-free: a caller may capture it in a
  * CUDA graph. */
 AXB_API int axb_batch_substep(axb_ctx *ctx, axb_batch *batch, double alpha,
