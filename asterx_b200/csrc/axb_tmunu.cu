@@ -48,11 +48,12 @@ AXB_D double c2v2(const double *__restrict__ f, long long I, long long sy, long 
   return s / 8.0;
 }
 
-// T_{mu nu} of the fluid interpolated to vertex I (rho, eps, press, B^i and
-// v^i or z^i), added to the arrays (tmunu.cxx:76-178).
-template <bool ZVEC>
-AXB_D void tmunu_point(const TmunuArgs &a, long long I, double rho_avg, double eps_avg,
-                       double press_avg, const double (&Bup)[3], const double (&vz)[3]) {
+// T_{mu nu} of the fluid at vertex I, added to the arrays (tmunu.cxx:76-178);
+// `field(v)` is field v of TmunuArgs::f interpolated there.
+template <bool ZVEC, class Field>
+AXB_D void tmunu_point(const TmunuArgs &a, long long I, const Field &field) {
+  const double rho_avg = field(0), eps_avg = field(1), press_avg = field(2);
+  const double Bup[3] = {field(3), field(4), field(5)};
   const sym3 g{__ldg(a.g[0] + I), __ldg(a.g[1] + I), __ldg(a.g[2] + I),
                __ldg(a.g[3] + I), __ldg(a.g[4] + I), __ldg(a.g[5] + I)};
   const double alp = __ldg(a.alp + I);
@@ -63,6 +64,7 @@ AXB_D void tmunu_point(const TmunuArgs &a, long long I, double rho_avg, double e
   const double beta_sq = dot3(beta_low, beta_up);
 
   double vup[3], vlow[3], w;
+  const double vz[3] = {field(6), field(7), field(8)};
   if constexpr (!ZVEC) {
     for (int d = 0; d < 3; ++d)
       vup[d] = vz[d];
@@ -113,22 +115,17 @@ AXB_D void tmunu_point(const TmunuArgs &a, long long I, double rho_avg, double e
     a.eT[c][I] = a.eT[c][I] + t[c];
 }
 
-// Order 2: one thread per interior vertex [ng, ng + n]; x along the block's
-// threads, the 8 cells around a vertex from L1/L2.
+// Order 2: one thread per interior vertex [ng, ng + n], a plane's vertices row
+// after row (rows of n + 1 cut into blocks of 128 leave the second block of
+// each with one thread at n = 128); the 8 cells around a vertex from L1/L2.
 template <bool ZVEC> __global__ void __launch_bounds__(128) k_tmunu2(const TmunuArgs a) {
   const BoxDev &b = a.b;
-  const int i = b.ng + blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = b.ng + blockIdx.y;
-  const int k = b.ng + blockIdx.z;
-  if (i > b.ng + b.n[0])
+  const int flat = blockIdx.x * blockDim.x + threadIdx.x, w = b.n[0] + 1;
+  const int row = flat / w;
+  if (row > b.n[1])
     return;
-  const long long I = b.at(i, j, k);
-  double q[9];
-#pragma unroll
-  for (int v = 0; v < 9; ++v)
-    q[v] = c2v2(a.f[v], I, b.sy, b.sz);
-  const double B[3] = {q[3], q[4], q[5]}, vz[3] = {q[6], q[7], q[8]};
-  tmunu_point<ZVEC>(a, I, q[0], q[1], q[2], B, vz);
+  const long long I = b.at(b.ng + flat - row * w, b.ng + row, b.ng + blockIdx.y);
+  tmunu_point<ZVEC>(a, I, [&](int v) { return c2v2(a.f[v], I, b.sy, b.sz); });
 }
 
 // Order 4: the cubic Lagrange weights (-1, 9, 9, -1)/16 on cells I-2 .. I+1
@@ -268,16 +265,18 @@ template <bool ZVEC> __global__ void __launch_bounds__(T4_N, 1) k_tmunu4(const T
   for (int q = 0; q < T4_Z; ++q) {
     if (k0 + q > b.ng + b.n[2])
       break;
-    auto res = [&](int v) { return s_res[(v * T4_Z + q) * T4_N]; };
-    const double B[3] = {res(3), res(4), res(5)}, vz[3] = {res(6), res(7), res(8)};
-    tmunu_point<ZVEC>(a, b.at(i, j, k0 + q), res(0), res(1), res(2), B, vz);
+    tmunu_point<ZVEC>(a, b.at(i, j, k0 + q),
+                      [&](int v) { return s_res[(v * T4_Z + q) * T4_N]; });
   }
 }
 
 template <bool ZVEC> int launch_tmunu(int order, const TmunuArgs &a, cudaStream_t s) {
   const int *n = a.b.n;
   if (order == 2) {
-    k_tmunu2<ZVEC><<<dim3((n[0] + 1 + 127) / 128, n[1] + 1, n[2] + 1), 128, 0, s>>>(a);
+    const long long plane = (long long)(n[0] + 1) * (n[1] + 1);
+    if (plane > 0x7fffff00LL)
+      return AXB_ERR_TOO_LARGE;
+    k_tmunu2<ZVEC><<<dim3(unsigned((plane + 127) / 128), n[2] + 1), 128, 0, s>>>(a);
     return AXB_OK;
   }
   if (cudaFuncSetAttribute(k_tmunu4<ZVEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
