@@ -45,7 +45,7 @@ int launch_sync_batch(const void *args, const TileTable &t, unsigned long long *
 int launch_c2p_batch(int which, const void *args, const TileTable &t,
                      unsigned long long *ctr, const axb_eos &eos, DevStatus *status,
                      int nblocks, cudaStream_t s, unsigned long long *queue = nullptr,
-                     int deferred_blocks = 0);
+                     int deferred_blocks = 0, bool noble = false);
 bool c2p_batch_fast_ok(int nbox, const axb_box *boxes, const axb_params *p);
 } // namespace axb
 
@@ -86,6 +86,7 @@ struct axb_batch {
   int nbox = 0;
   int sms = 148;
   int recon = 0, fd_order = 2;
+  bool noble = false; // Noble is the first solver
   const axb_eos *eos = nullptr;
   DevStatus *status = nullptr;
   void *rhs_args = nullptr, *c2p_args = nullptr;
@@ -190,7 +191,7 @@ int launch_phase(axb_ctx *c, const axb_batch *B, int phase, const BatchStage &st
   case P_BSTAG: rc = launch_c2p_batch(0, B->c2p_args, t, ctr, *B->eos, B->status, nb, s); break;
   case P_C2P:
     rc = launch_c2p_batch(1, B->c2p_args, t, ctr, *B->eos, B->status, nb, s, B->c2p_queue,
-                          4 * B->sms);
+                          4 * B->sms, B->noble);
     break;
   case P_SYNC_P: rc = launch_sync_batch(B->sync_p, t, ctr, nb, s); break;
   }
@@ -242,6 +243,7 @@ AXB_API int axb_batch_create(axb_ctx *c, int nbox, const axb_box *boxes,
   B->nbox = nbox;
   B->recon = p->reconstruction_method;
   B->fd_order = p->local_spatial_order;
+  B->noble = p->c2p_prime == AXB_C2P_NOBLE;
   B->eos = eos;
   B->status = c->status;
   for (int ph = 0; ph < NPHASE; ++ph)

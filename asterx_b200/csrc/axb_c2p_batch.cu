@@ -30,6 +30,13 @@ __global__ void __launch_bounds__(128, AXB_C2P_MINB)
     k_c2p_deferred_batch(const C2PBoxArgs *args, const __grid_constant__ EOS eos, const C2PQueue q) {
   c2p_deferred_body([&](int box) -> const C2PBoxArgs & { return args[box]; }, eos, q);
 }
+__global__ void __launch_bounds__(128, NOBLE_MINB)
+    k_c2p_noble_batch(const C2PBoxArgs *args, const TileTable t, unsigned long long *ctr,
+                      const __grid_constant__ EosIdeal eos) {
+  batch_loop(args, t, ctr, [&](const C2PBoxArgs &a, const uint3 bid) {
+    c2p_noble_body<false>(a, eos, bid);
+  });
+}
 template <class EOS>
 int launch_c2p_batch_eos(const C2PBoxArgs *a, const TileTable &t, unsigned long long *ctr,
                          const EOS &eos, int nblocks, unsigned long long *queue,
@@ -85,12 +92,12 @@ uint3 c2p_grid(int which, const axb_box &b) {
 }
 
 // `queue` (count, then room for every interior cell of the batch) selects
-// the fast pass + deferred full cascade (Palenzuela first), else the full
-// cascade in one launch.
+// the fast pass + deferred full cascade (Palenzuela first), else Noble's
+// kernel (`noble`, ideal gas) or the full cascade in one launch.
 int launch_c2p_batch(int which, const void *args, const TileTable &t,
                      unsigned long long *ctr, const axb_eos &eos, DevStatus *status,
                      int nblocks, cudaStream_t s, unsigned long long *queue,
-                     int deferred_blocks) {
+                     int deferred_blocks, bool noble) {
   if (t.total == 0)
     return AXB_OK;
   const C2PBoxArgs *a = static_cast<const C2PBoxArgs *>(args);
@@ -101,6 +108,10 @@ int launch_c2p_batch(int which, const void *args, const TileTable &t,
   if (eos.kind == 1)
     return launch_c2p_batch_eos(a, t, ctr, tab_for_launch(eos, status), nblocks, queue,
                                 deferred_blocks, s);
+  if (noble) {
+    k_c2p_noble_batch<<<nblocks, 128, 0, s>>>(a, t, ctr, eos.ideal);
+    return cudaGetLastError() == cudaSuccess ? AXB_OK : AXB_ERR_CUDA;
+  }
   return launch_c2p_batch_eos(a, t, ctr, eos.ideal, nblocks, queue, deferred_blocks, s);
 }
 

@@ -290,6 +290,42 @@ AXB_D GuessStart guess_start(const C2PBoxArgs &a, int i, int j, int k, const Cel
   return g;
 }
 
+// The first solver's seeds: the saved primitives, their velocity limited
+// (con2prim.cxx:168-229).
+template <class EOS>
+AXB_D void c2p_seeds(const C2PBoxArgs &a, const EOS &eos, const CellData &c, Prim &seeds) {
+  const long long I = c.I;
+  double v_up[3] = {a.saved_vel[0][I], a.saved_vel[1][I], a.saved_vel[2][I]};
+  double v_low[3];
+  lower3(c.glo, v_up, v_low);
+  double zsq;
+  const double vsq = dot3(v_low, v_up);
+  if (vsq >= 1.0) {
+    const double wlim = sqrt(1.0 + a.cp.vw_lim * a.cp.vw_lim);
+    const double vlim = a.cp.vw_lim / wlim;
+    for (int q = 0; q < 3; ++q)
+      v_up[q] *= vlim / sqrt(vsq);
+    zsq = a.cp.vw_lim * a.cp.vw_lim;
+  } else {
+    zsq = vsq / (1.0 - vsq);
+  }
+  seeds.rho = a.saved_rho[I];
+  seeds.eps = a.saved_eps[I];
+  seeds.Ye = a.saved_Ye[I];
+  {
+    double e = seeds.eps; // the reference clamps a copy, not the seed
+    seeds.press = eos.press_from_valid_rho_eps_ye(seeds.rho, e, seeds.Ye);
+  }
+  seeds.temperature = a.temperature[I];
+  seeds.entropy = 0.0; // only read by the excision path, filled there
+  for (int q = 0; q < 3; ++q) {
+    seeds.vel[q] = v_up[q];
+    seeds.Bvec[q] = c.Bup[q];
+    seeds.E[q] = 0.0;
+  }
+  seeds.w_lor = sqrt(1.0 + zsq);
+}
+
 // One cell of AsterX_Con2Prim_typeEoS (con2prim.cxx:81-453), the whole
 // cascade.
 //
@@ -309,40 +345,10 @@ AXB_D int c2p_cell(const C2PBoxArgs &a, const EOS &eos, const int i, const int j
   const sym3 &glo = c.glo;
   Cons &cv = c.cv;
   double mask_local = 1.0;
-  double v_up[3] = {a.saved_vel[0][I], a.saved_vel[1][I], a.saved_vel[2][I]};
-  double v_low[3];
-  lower3(glo, v_up, v_low);
-  double zsq;
-  const double vsq = dot3(v_low, v_up);
-  if (vsq >= 1.0) {
-    const double wlim = sqrt(1.0 + a.cp.vw_lim * a.cp.vw_lim);
-    const double vlim = a.cp.vw_lim / wlim;
-    for (int q = 0; q < 3; ++q) {
-      v_up[q] *= vlim / sqrt(vsq);
-      v_low[q] *= vlim / sqrt(vsq);
-    }
-    zsq = a.cp.vw_lim * a.cp.vw_lim;
-  } else {
-    zsq = vsq / (1.0 - vsq);
-  }
   Prim pv;
   pv.set_nan();
   Prim seeds;
-  seeds.rho = a.saved_rho[I];
-  seeds.eps = a.saved_eps[I];
-  seeds.Ye = a.saved_Ye[I];
-  {
-    double e = seeds.eps; // the reference clamps a copy, not the seed
-    seeds.press = eos.press_from_valid_rho_eps_ye(seeds.rho, e, seeds.Ye);
-  }
-  seeds.temperature = a.temperature[I];
-  seeds.entropy = 0.0; // only read by the excision path, filled there
-  for (int q = 0; q < 3; ++q) {
-    seeds.vel[q] = v_up[q];
-    seeds.Bvec[q] = c.Bup[q];
-    seeds.E[q] = 0.0;
-  }
-  seeds.w_lor = sqrt(1.0 + zsq);
+  c2p_seeds(a, eos, c, seeds);
   bool flag_local = true;
   int code = AXB_C2P_INIT;
   bool call_c2p = true;
@@ -461,6 +467,69 @@ template <class EOS, bool GUESS = false>
 __global__ void __launch_bounds__(128, AXB_C2P_MINB)
     k_c2p_box(const C2PBoxArgs a, const __grid_constant__ EOS eos) {
   c2p_box_body<EOS, GUESS>(a, eos, blockIdx);
+}
+
+// Noble first on the ideal gas: the first solver's common path alone, whose
+// values fit the registers of NOBLE_MINB CTAs per SM where the whole cascade's
+// spilled; a cell that needs anything else (inside the mask, or a failed Noble search)
+// calls the cascade, out of line and with nothing written.  No queue and no
+// second launch, which small boxes would wait for.  190x131x162 cells 824 ->
+// 590 us (5 CTAs per SM 597, 6: 733, 8: 893), 96^3 195 -> 144 us, 30x39x52 35 ->
+// 15 us.
+constexpr int NOBLE_MINB = 4;
+template <bool GUESS>
+__device__ __noinline__ void c2p_cascade(const C2PBoxArgs &a, const EosIdeal &eos, int i, int j,
+                                         int k, int &iters_first, bool &failed) {
+  c2p_cell_full<EosIdeal, GUESS>(a, eos, i, j, k, iters_first, failed);
+}
+template <bool GUESS>
+AXB_D void c2p_noble_body(const C2PBoxArgs &a, const EosIdeal &eos, const uint3 bid) {
+  __shared__ unsigned int s_hist[64];
+  c2p_hist_init(a, s_hist);
+  int i, j;
+  const int k = a.b.ng + bid.z;
+  int iters_first = -1;
+  bool failed = false;
+  if (a.b.row_ij(a.b.ng, a.b.n[0], a.b.ng, a.b.n[1], bid, i, j)) {
+    CellData c;
+    c2p_gather(a, eos, i, j, k, c);
+    bool rare = c.alp_avg < a.cp.alp_thresh;
+    if (!rare) {
+      Prim pv;
+      int code = AXB_C2P_PRIME;
+      if (c.cv.dens <= c.sqrt_detg * c.atmo.rho_cut) {
+        for (int d = 0; d < 3; ++d)
+          pv.Bvec[d] = c.Bup[d];
+        c.atmo.set(pv, c.cv, c.glo);
+        cons_floors(c.cv, c.glo);
+        code = AXB_C2P_ATMO;
+      } else {
+        Prim seeds;
+        c2p_seeds(a, eos, c, seeds);
+        GuessStart g;
+        if constexpr (GUESS)
+          g = guess_start(a, i, j, k, c);
+        cons_floors(c.cv, c.glo);
+        Report rep;
+        noble_solve(eos, a.cp, c.atmo, a.gamma_noble, a.Zmin, pv, seeds, c.cv, c.glo, rep, g.z,
+                    g.vsq);
+        rare = rep.failed();
+        iters_first = rep.iters;
+      }
+      if (!rare)
+        c2p_store(a, c.I, code, pv, c.cv);
+    }
+    if (rare) {
+      iters_first = -1;
+      c2p_cascade<GUESS>(a, eos, i, j, k, iters_first, failed);
+    }
+  }
+  c2p_epilogue(a, s_hist, iters_first, failed);
+}
+template <bool GUESS>
+__global__ void __launch_bounds__(128, NOBLE_MINB)
+    k_c2p_noble(const __grid_constant__ C2PBoxArgs a, const __grid_constant__ EosIdeal eos) {
+  c2p_noble_body<GUESS>(a, eos, blockIdx);
 }
 
 // Deferred cells of a fast pass: the count, then one entry per cell,

@@ -218,6 +218,8 @@ void launch_box_recovery(const C2PBoxArgs &a, const axb_eos *eos, const dim3 gri
     }
   } else if (eos->kind == 1) {
     k_c2p_box<EosTab, GUESS><<<grid, T, 0, s>>>(a, tab_for_launch(*eos, a.status));
+  } else if (a.c2p_prime == AXB_C2P_NOBLE) {
+    k_c2p_noble<GUESS><<<grid, T, 0, s>>>(a, eos->ideal);
   } else {
     k_c2p_box<EosIdeal, GUESS><<<grid, T, 0, s>>>(a, eos->ideal);
   }
