@@ -94,7 +94,10 @@ struct EosTab {
   // the trilinear interpolant, along ln rho, then ln T, then Ye
   AXB_HD double tri(int var, const Cell &c, double lt) const {
     const int j = find(1, lt);
-    const double w = (lt - x[1][j]) / (x[1][j + 1] - x[1][j]);
+    return tri_in(var, c, j, (lt - x[1][j]) / (x[1][j + 1] - x[1][j]));
+  }
+  // the same with the T cell and the weight in it given
+  AXB_HD double tri_in(int var, const Cell &c, int j, double w) const {
     double B[2];
 #pragma unroll
     for (int o = 0; o < 2; ++o) {
@@ -280,8 +283,14 @@ struct EosTab {
   // eps, press and the product of two sound-speed queries of a face state
   // given by its temperature (fluxes.cxx:297-304,556-560): eps from the
   // clamped logarithms, press from the plain ones, as the two queries take
-  // them; cs^2 at that eps, found from the temperature's own cell.  eps2 is
-  // eps as the sound-speed query leaves it (it may clamp).
+  // them; cs^2 at that eps.  eps2 is eps as the sound-speed query leaves it (it
+  // may clamp).
+  //
+  // The sound-speed query inverts eps for the temperature eps came from.  Where
+  // the state lies inside the table and eps grows with T there, that is the
+  // temperature at hand, so cs^2 is read at it: no logarithm, node search,
+  // root or product of square roots (96^3 RHS 2.36 -> 2.01 ms), and without the
+  // rounding the inversion amplifies where eps hardly depends on T.
   struct FaceThermo {
     double eps, press, cs2, eps2;
   };
@@ -291,13 +300,23 @@ struct EosTab {
     const double T = fmin(fmax(temp, rgtemp.min), rgtemp.max);
     const double lr = log(r), lt = log(T);
     const Cell c = locate(lr, ye);
-    o.eps = exp(tri(TAB_EPS, c, lt)) - shift;
-    if (r == rho && T == temp)
-      o.press = exp(tri(TAB_PRESS, c, lt));
+    const int j = find(1, lt);
+    const double w = (lt - x[1][j]) / (x[1][j + 1] - x[1][j]);
+    o.eps = exp(tri_in(TAB_EPS, c, j, w)) - shift;
+    const bool plain = r == rho && T == temp;
+    if (plain)
+      o.press = exp(tri_in(TAB_PRESS, c, j, w));
     else
       o.press = exp(tri(TAB_PRESS, locate(log(rho), ye), log(temp)));
+    if (plain && monotone && o.eps >= rgeps.min && c.u >= 0.0 && c.u <= 1.0 && c.v >= 0.0 &&
+        c.v <= 1.0 && w >= 0.0 && w <= 1.0) {
+      o.eps2 = (o.eps + shift) - shift;
+      o.cs2 = tri_in(TAB_CS2, c, j, w);
+      if (o.cs2 >= 0.0)
+        return o; // else NaN, as the root below gives it
+    }
     o.eps2 = o.eps;
-    int hint = find(1, lt);
+    int hint = j;
     const double cs = sqrt(tri(TAB_CS2, c, logtemp_at(c, lr, o.eps2, ye, hint)));
     o.cs2 = cs * cs;
     if (!(o.eps2 == o.eps))
