@@ -365,25 +365,36 @@ AXB_HD void set_E(Prim &pv, const sym3 &gup) {
 }
 
 // The Newton search of the Noble scheme (c2p_2DNoble.hxx:404-515) in (Z, v^2)
-// from undensitised D, E = tau + D, S^2, B^2 and B.S; gg = (Gamma-1)/Gamma.
-// A step takes two divisions and one reciprocal square root where the
-// reference's expressions take seven divisions and a square root (FP64
-// divisions were most of a step's time): the divisions by Gamma become one
-// product with gg, sqrt(1-v^2) and its reciprocal come from one rsqrt, the
-// determinant is formed from the Jacobian's terms, |dx/x| <= tol is tested as
-// |dx| <= tol |x|, and multiply-adds are explicit.  Last-ulp differences in a
-// search that converges quadratically to tol.
+// from undensitised D, tau, S^2, B^2 and B.S; gg = (Gamma-1)/Gamma.
+//
+// CHEAP, for the kernels that take Noble's common path: a step takes two
+// divisions and one reciprocal square root where the reference's expressions
+// take seven divisions and a square root (FP64 divisions were most of a step's
+// time): the divisions by Gamma become one product with gg, sqrt(1-v^2) and
+// its reciprocal come from one rsqrt, the determinant is formed from the
+// Jacobian's terms, |dx/x| <= tol is tested as |dx| <= tol |x|, and
+// multiply-adds are explicit.  Last-ulp differences in a search that converges
+// quadratically to tol.
+//
+// Otherwise the reference's expressions, for the cascade: the cells it gets
+// are the hard ones, whose last steps are rounding noise about the size of
+// tol, and whether such a search ends within max_iter must not depend on a
+// last ulp (1e-5 of the cells of a box with W <= 10 and max_iter = 30 took
+// another flag with the cheaper step).
 struct NobleRoot {
   double Z, vsq;
   int iters;
   bool slow;   // not converged within max_iter
   bool finite; // the last residual is finite
 };
-AXB_HD NobleRoot noble_root(double D, double E, double Ssq, double Bsq, double BiSi, double gg,
-                            double Zmin, double tol, int max_iter, double x0, double x1) {
+template <bool CHEAP>
+AXB_HD NobleRoot noble_root(double D, double tau, double Ssq, double Bsq, double BiSi,
+                            double gamma, double gg, double Zmin, double tol, int max_iter,
+                            double x0, double x1) {
   constexpr double dv = (1. - 1.e-10);
-  const double b2 = BiSi * BiSi, hB = 0.5 * Bsq;
   double xo0 = x0, err = 1.0, lim = 0.0, r0 = 0.0, r1 = 0.0;
+  if constexpr (!CHEAP)
+    lim = tol;
   if (x1 < 0.0)
     x1 = 0.0;
   else if (x1 >= 1.0)
@@ -395,21 +406,44 @@ AXB_HD NobleRoot noble_root(double D, double E, double Ssq, double Bsq, double B
   int k;
   for (k = 1; k <= max_iter; ++k) {
     const double Z = x0, V = x1;
-    const double iZ = 1.0 / Z;
-    const double om = 1.0 - V;
-    const double is = rsqrt(om);
-    const double ZB = Bsq + Z, ZB2 = ZB * ZB;
-    const double b2z2 = b2 * iZ * iZ, Vb = fma(b2z2, iZ, V); // v^2 + (B.S)^2 / Z^3
-    const double p = fma(Z, om, -D * (om * is)) * gg;        // P(Z, v^2)
-    const double dPv = fma(0.5 * D, is, -Z) * gg;
-    const double fj00 = -2.0 * Vb * ZB;
-    const double fj10 = fma(om, gg, -1.0) - (Vb - V);
-    const double fj11 = dPv - hB;
-    r0 = fma(b2z2, ZB + Z, fma(-V, ZB2, Ssq));
-    r1 = (fma(0.5, b2z2, fma(-hB, 1.0 + V, E)) - Z) + p;
-    const double idet = 1.0 / fma(fj10, ZB2, fj00 * fj11);
-    const double dx0 = -fma(fj11, r0, ZB2 * r1) * idet;
-    const double dx1 = -fma(-fj10, r0, fj00 * r1) * idet;
+    double dx0, dx1;
+    if constexpr (CHEAP) {
+      const double b2 = BiSi * BiSi, hB = 0.5 * Bsq;
+      const double iZ = 1.0 / Z;
+      const double om = 1.0 - V;
+      const double is = rsqrt(om);
+      const double ZB = Bsq + Z, ZB2 = ZB * ZB;
+      const double b2z2 = b2 * iZ * iZ, Vb = fma(b2z2, iZ, V); // v^2 + (B.S)^2 / Z^3
+      const double p = fma(Z, om, -D * (om * is)) * gg;        // P(Z, v^2)
+      const double dPv = fma(0.5 * D, is, -Z) * gg;
+      const double fj00 = -2.0 * Vb * ZB;
+      const double fj10 = fma(om, gg, -1.0) - (Vb - V);
+      const double fj11 = dPv - hB;
+      r0 = fma(b2z2, ZB + Z, fma(-V, ZB2, Ssq));
+      r1 = (fma(0.5, b2z2, fma(-hB, 1.0 + V, tau + D)) - Z) + p;
+      const double idet = 1.0 / fma(fj10, ZB2, fj00 * fj11);
+      dx0 = -fma(fj11, r0, ZB2 * r1) * idet;
+      dx1 = -fma(-fj10, r0, fj00 * r1) * idet;
+    } else {
+      const double gfac = gamma - 1.0;
+      const double invZ = 1.0 / Z;
+      const double Sdotn = -(tau + D);
+      const double p_tmp = ((Z * (1.0 - V) - D * sqrt(1.0 - V)) * gfac / (gamma));
+      const double dPdvsq = ((-Z + D / (2.0 * sqrt(1.0 - V))) * gfac / gamma);
+      const double dPdZ = ((1.0 - V) * gfac / gamma);
+      const double fj00 = -2 * (V + BiSi * BiSi * invZ * invZ * invZ) * (Bsq + Z);
+      const double fj01 = -(Bsq + Z) * (Bsq + Z);
+      const double fj10 = -1.0 + dPdZ - BiSi * BiSi * invZ * invZ * invZ;
+      const double fj11 = -0.5 * Bsq + dPdvsq;
+      r0 = Ssq - V * (Bsq + Z) * (Bsq + Z) + BiSi * BiSi * invZ * invZ * (Bsq + Z + Z);
+      r1 = -Sdotn - 0.5 * Bsq * (1.0 + V) + 0.5 * BiSi * BiSi * invZ * invZ - Z + p_tmp;
+      const double detjac = (Bsq + Z) * (fj10 * (Bsq + Z) + (Bsq - 2.0 * dPdvsq) *
+                                                              (BiSi * BiSi * invZ * invZ + V * Z) *
+                                                              invZ);
+      const double detjac_inv = 1.0 / detjac;
+      dx0 = -(fj11 * r0 - fj01 * r1) * detjac_inv;
+      dx1 = -(-fj10 * r0 + fj00 * r1) * detjac_inv;
+    }
     xo0 = x0;
     x0 += dx0;
     x1 += dx1;
@@ -421,8 +455,12 @@ AXB_HD NobleRoot noble_root(double D, double E, double Ssq, double Bsq, double B
       x0 = fabs(x0) + Zmin;
     else if (x0 > 1e20)
       x0 = xo0;
-    err = fabs(dx0);
-    lim = x0 == 0.0 ? tol : tol * fabs(x0);
+    if constexpr (CHEAP) {
+      err = fabs(dx0);
+      lim = x0 == 0.0 ? tol : tol * fabs(x0);
+    } else {
+      err = (x0 == 0.) ? fabs(dx0) : fabs(dx0 / x0);
+    }
     if (err <= lim)
       break;
   }
@@ -436,7 +474,7 @@ AXB_HD NobleRoot noble_root(double D, double E, double Ssq, double Bsq, double B
 // Seeds (rho, eps, Ye, vel) come in pv_seeds; `zguess` >= 0 replaces the
 // Z seed and `vsqguess` in [0,1) the v^2 seed (learned initial guess).
 // ---------------------------------------------------------------------------
-template <class EOS>
+template <class EOS, bool CHEAP = false>
 AXB_HD void noble_solve(const EOS &eos, const C2PParams &cp, const Atmo &atmo,
                         double gamma, double Zmin, Prim &pv, Prim &pv_seeds,
                         Cons &cv, const sym3 &glo, Report &rep,
@@ -507,8 +545,9 @@ AXB_HD void noble_solve(const EOS &eos, const C2PParams &cp, const Atmo &atmo,
     x0 = zguess;
     x1 = vsqguess;
   }
-  const NobleRoot root = noble_root(cv.dens, cv.tau + cv.dens, Ssq, Bsq, BiSi,
-                                    (gamma - 1.0) / gamma, Zmin, cp.tol, cp.maxIter, x0, x1);
+  const NobleRoot root =
+      noble_root<CHEAP>(cv.dens, cv.tau, Ssq, Bsq, BiSi, gamma, (gamma - 1.0) / gamma, Zmin,
+                        cp.tol, cp.maxIter, x0, x1);
   rep.iters = root.iters;
   if (root.slow) {
     rep.fail(REP_ROOT_FAIL_CONV);

@@ -511,8 +511,8 @@ AXB_D void c2p_noble_body(const C2PBoxArgs &a, const EosIdeal &eos, const uint3 
           g = guess_start(a, i, j, k, c);
         cons_floors(c.cv, c.glo);
         Report rep;
-        noble_solve(eos, a.cp, c.atmo, a.gamma_noble, a.Zmin, pv, seeds, c.cv, c.glo, rep, g.z,
-                    g.vsq);
+        noble_solve<EosIdeal, true>(eos, a.cp, c.atmo, a.gamma_noble, a.Zmin, pv, seeds, c.cv,
+                                    c.glo, rep, g.z, g.vsq);
         rare = rep.failed();
         iters_first = rep.iters;
       }
@@ -571,7 +571,8 @@ AXB_D void queue_deferred(const C2PQueue &q, bool defer, int i, int j, int k, in
 // the same whichever thread runs them.  A table's step (an inversion and
 // three logarithms or exponentials) is long enough to pay for it: 96^3 cells
 // 9.2 -> 2.7 ms together with the queries as function calls from a temperature
-// cell kept between steps (6 / 10 first and 6 further steps: the same).  An
+// cell kept between steps (6 / 10 first and 6 further steps: the same; 2.38 ms
+// with the plane's rows laid end to end).  An
 // ideal gas's step is not: 4.0M cells 1.24 ms one cell per thread, 1.46 ms
 // through the pool even without a second round (its records and barriers),
 // 1.51 ms with rounds.

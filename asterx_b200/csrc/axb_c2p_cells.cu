@@ -336,8 +336,9 @@ __global__ void __launch_bounds__(128, 8)
         x0 = fabs(D * W * (1.0 + eps + eos.gm1 * eps));
         x1 = vsq;
       }
-      const NobleRoot r = noble_root(D, tau + D, Ssq, Bsq, BiSi, a.gfac_over_gamma, a.Zmin,
-                                     a.cp.tol, a.cp.maxIter, x0, x1);
+      const NobleRoot r =
+          noble_root<true>(D, tau, Ssq, Bsq, BiSi, a.gamma_noble, a.gfac_over_gamma, a.Zmin,
+                           a.cp.tol, a.cp.maxIter, x0, x1);
       common = !r.slow && r.finite;
       if (common) {
         // WZ2Prim (c2p_2DNoble.hxx:192-273): W = (1 - v^2)^-1/2, rho = D / W,
