@@ -31,8 +31,9 @@ struct BoxDev {
   double dx[3], idx[3];
   double xmin[3];
   // 0: a block covers one row (block x along i, bid.y = j); 1 (batched
-  // launches over small boxes): the blocks of a k-plane cover its (i, j)
-  // points row after row, so short rows do not leave threads idle
+  // launches, and a box where it takes fewer blocks): the blocks of a k-plane
+  // cover its (i, j) points row after row, so short rows do not leave threads
+  // idle
   int packed;
 
   // the (i, j) of this thread for a range [li, li + ni) x [lj, lj + nj);

@@ -223,7 +223,8 @@ AXB_D void cp_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory")
 // three CTAs per SM fit, whose 168 registers hold both face states without
 // spills (four at 128 registers spilled, and kept the left state in shared
 // memory).  256^3 WENO-Z: y 3.55 -> 2.87 ms, z 3.80 -> 3.09 ms (beside the
-// sources).  Not kept: a four-slot ring with the last row loaded directly at
+// sources; with fold_divergence's loads ahead of its stores, and the z pass's
+// in two batches from U prefetched, 2.52 and 2.49 ms).  Not kept: a four-slot ring with the last row loaded directly at
 // four CTAs (3.05 / 3.31 ms) or three (2.95 / 3.09); seven 64-thread CTAs at
 // 128 registers (3.39 / 3.66).
 // Transverse range: cells [ng-1, ng+n] (one ghost layer each side, needed
