@@ -199,7 +199,10 @@ int launch_phase(axb_ctx *c, const axb_batch *B, int phase, const BatchStage &st
   return rc;
 }
 
+// one RHS evaluation, stored.  Every round of launches starts from zeroed work
+// counters: a tile drawn from a counter that was never set can be negative
 int run_rhs_phases(axb_ctx *c, const axb_batch *B, cudaStream_t s) {
+  AXB_CUDA_TRY(cudaMemsetAsync(B->ctr, 0, NPHASE * sizeof(unsigned long long), s));
   for (int ph = P_SOURCES; ph <= P_CT; ++ph) {
     const int rc = launch_phase(c, B, ph, BatchStage{}, s);
     if (rc)

@@ -10,7 +10,7 @@ import pytest
 
 from asterx_b200 import abi
 from asterx_b200 import workloads as W
-from tests.helpers import full_fields
+from tests.helpers import errors, full_fields, interior
 
 SSPRK3 = [(0.0, 1.0, 1.0), (0.75, 0.25, 0.25), (1.0 / 3.0, 2.0 / 3.0, 2.0 / 3.0)]
 SHAPES = [(12, 10, 8), (8, 8, 8), (16, 8, 12), (10, 14, 9), (9, 9, 9), (20, 6, 7)]
@@ -103,6 +103,39 @@ def test_batch_matches_per_box(engine, recon):
                     sc = np.nanmax(np.abs(x)) or 1.0
                     assert np.nanmax(np.abs(x - y)) <= 1e-9 * sc, (tune, q, k)
         engine.batch_destroy(batch)
+
+
+@pytest.mark.gpu
+def test_autotune_of_a_new_batch(engine):
+    """The autotuner as the first call on a batch whose device blocks come from
+    memory that held negative numbers: its work counters are its own to zero
+    (a negative one names a tile before the first), and it leaves one RHS
+    evaluation behind (<= 1e-12 of the largest value, as the RHS parity tests)."""
+    import ctypes as C
+    cudart = C.CDLL("libcudart.so.12")
+    blocks = []
+    for size in [64, 128, 256, 512, 1024, 4096] * 32:
+        q = C.c_void_p()
+        assert cudart.cudaMalloc(C.byref(q), C.c_size_t(size)) == 0
+        assert cudart.cudaMemset(q, 0xFF, C.c_size_t(size)) == 0
+        blocks.append(q)
+    for q in blocks:
+        assert cudart.cudaFree(q) == 0
+    boxes = make_boxes(engine)
+    p = abi.default_params(reconstruction_method="wenoz", flux_type="hlle",
+                           c2p_prime="palenzuela", c2p_second="noble")
+    eos = engine.eos_idealgas(4.0 / 3.0, rho=(1e-40, 1e10), eps=(0.0, 1e10))
+    dev, devn = upload(engine, boxes)
+    batch = engine.batch_create([L for L, _ in boxes], dev, devn, p, eos)
+    engine.batch_autotune(batch)
+    for (L, f), d in zip(boxes, dev):
+        one = engine.upload(L, f)
+        engine.rhs_group(L, one, p, eos)
+        for k in abi.HYDRO_RHS + abi.AVEC_RHS:
+            emax, _ = errors(interior(L, k, d[k].cpu().numpy()),
+                             interior(L, k, one[k].cpu().numpy()))
+            assert emax <= 1e-12, (L.n, k, emax)
+    engine.batch_destroy(batch)
 
 
 @pytest.mark.gpu
