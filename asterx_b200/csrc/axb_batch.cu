@@ -7,9 +7,9 @@
 // tiles of all boxes (axb_batch.cuh), the per-box argument blocks live in
 // device memory, and the whole substep (11 launches plus one memset of the
 // work counters) is stream-ordered and allocation-free, so a caller can
-// capture it in a CUDA graph.  The autotuner picks the pencil segment length
-// of the y and z flux passes and the number of resident CTAs per SM of the
-// persistent grids by timing them on the batch's own boxes.
+// capture it in a CUDA graph.  The pencil segments of the y and z flux passes
+// follow from the level's size; the autotuner checks them, and the number of
+// resident CTAs per SM of the persistent grids, by timing the batch's own boxes.
 #include <algorithm>
 #include <cstring>
 #include <new>
@@ -93,7 +93,8 @@ struct axb_batch {
   void *sync_e = nullptr, *sync_p = nullptr;
   DevTable tab[NPHASE];
   // y, z tables: the autotuner's candidate segments, then the one chosen by
-  // the level's size (split_steps), which stands until the autotuner is asked
+  // the level's size (split_steps), which stands unless the autotuner finds
+  // one of the others faster
   DevTable flux_seg[2][NSEG + 1];
   int steps[2] = {16, 16}; // that segment
   int seg[2] = {NSEG, NSEG}; // index of the table in use
@@ -319,13 +320,15 @@ AXB_API int axb_batch_substep(axb_ctx *c, axb_batch *B, double alpha, double bet
 }
 
 // Autotuner: times the RHS phases on the batch's own boxes for every
-// candidate pencil segment of the y and z flux passes and every candidate
-// persistent-grid size, and keeps the fastest of each.  The RHS phases
-// overwrite what they read back (sources and the x pass write, y and z
-// accumulate on top), so repeating them leaves the state as one RHS
-// evaluation would; the stage update and the post-step are not touched.
+// candidate persistent-grid size and every candidate pencil segment of the y
+// and z flux passes (the one axb_batch_create chose by the level's size is the
+// first of them), the best of three samples each, and keeps the fastest.  The
+// RHS phases overwrite what they read back (sources and the x pass write, y
+// and z accumulate on top; timed storing the RHS, not with the stage update
+// the substep makes in their place), so repeating them leaves the state as one
+// RHS evaluation would; the stage update and the post-step are not touched.
 // Synchronous; call it outside any stream capture.  out[0..1] receive the
-// chosen y / z segments, out[2] the chosen CTAs per SM of the flux passes.
+// y / z segments in use, out[2] the CTAs per SM of the flux passes.
 AXB_API int axb_batch_autotune(axb_ctx *c, axb_batch *B, int *out, void *stream) {
   if (!c || !B)
     return AXB_ERR_ARG;
@@ -335,19 +338,24 @@ AXB_API int axb_batch_autotune(axb_ctx *c, axb_batch *B, int *out, void *stream)
   AXB_CUDA_TRY(cudaEventCreate(&e1));
   const int saved_timing = c->timing;
   c->timing = 0;
-  auto time_rhs = [&](int phase, float &ms) -> int {
-    AXB_CUDA_TRY(cudaMemsetAsync(B->ctr, 0, NPHASE * sizeof(unsigned long long), s));
-    for (int ph = P_SOURCES; ph <= P_CT; ++ph) {
-      if (ph == phase)
-        AXB_CUDA_TRY(cudaEventRecord(e0, s));
-      const int rc = launch_phase(c, B, ph, BatchStage{}, s);
-      if (rc)
-        return rc;
-      if (ph == phase)
-        AXB_CUDA_TRY(cudaEventRecord(e1, s));
+  auto time_rhs = [&](int phase, float &best_ms) -> int {
+    best_ms = 1e30f;
+    for (int sample = 0; sample < 3; ++sample) {
+      AXB_CUDA_TRY(cudaMemsetAsync(B->ctr, 0, NPHASE * sizeof(unsigned long long), s));
+      for (int ph = P_SOURCES; ph <= P_CT; ++ph) {
+        if (ph == phase)
+          AXB_CUDA_TRY(cudaEventRecord(e0, s));
+        const int rc = launch_phase(c, B, ph, BatchStage{}, s);
+        if (rc)
+          return rc;
+        if (ph == phase)
+          AXB_CUDA_TRY(cudaEventRecord(e1, s));
+      }
+      float ms = 0;
+      AXB_CUDA_TRY(cudaEventSynchronize(e1));
+      AXB_CUDA_TRY(cudaEventElapsedTime(&ms, e0, e1));
+      best_ms = std::min(best_ms, ms);
     }
-    AXB_CUDA_TRY(cudaEventSynchronize(e1));
-    AXB_CUDA_TRY(cudaEventElapsedTime(&ms, e0, e1));
     return AXB_OK;
   };
   int rc = run_rhs_phases(c, B, s); // warm-up
@@ -368,9 +376,9 @@ AXB_API int axb_batch_autotune(axb_ctx *c, axb_batch *B, int *out, void *stream)
   }
   // segment length of the y and z passes
   for (int d = 0; d < 2 && !rc; ++d) {
-    int best = 0;
+    int best = B->seg[d] = NSEG; // the level's own choice is a candidate too
     float best_ms = 1e30f;
-    for (int q = 0; q < NSEG && !rc; ++q) {
+    for (int q = NSEG; q >= 0 && !rc; --q) {
       B->seg[d] = q;
       float ms = 0;
       rc = time_rhs(P_FLUX_Y + d, ms);
@@ -393,8 +401,8 @@ AXB_API int axb_batch_autotune(axb_ctx *c, axb_batch *B, int *out, void *stream)
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (out) {
-    out[0] = kSeg[B->seg[0]];
-    out[1] = kSeg[B->seg[1]];
+    out[0] = segment_of(B, 0);
+    out[1] = segment_of(B, 1);
     out[2] = B->ctas[P_FLUX_Y];
   }
   return rc;

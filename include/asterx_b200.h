@@ -457,12 +457,14 @@ AXB_API int axb_batch_substep(axb_ctx *ctx, axb_batch *batch, double alpha,
                               double beta, double gamma, double dt, int periodic,
                               void *stream);
 
-/* Autotuner: times the RHS phases on the batch's own boxes for pencil
- * segments {8, 16, 32, 64} of the y and z flux passes and persistent grids
- * of {2, 4, 8, 16} CTAs per SM, and keeps the fastest.  Leaves the RHS grid
- * functions as one RHS evaluation would.  Synchronous; not for use inside a
- * stream capture.  out (may be NULL, 3 ints): y segment, z segment, CTAs per
- * SM of the flux passes.  No counterpart in the reference. */
+/* Autotuner: times the RHS phases (storing the RHS) on the batch's own boxes
+ * for pencil segments of the y and z flux passes -- the one chosen by the
+ * level's size at creation (1 to 32 cells), 8, 16, 32 and 64 -- and persistent
+ * grids of {2, 4, 8, 16} CTAs per SM, three samples each, and keeps the
+ * fastest.  Leaves the RHS grid functions as one RHS evaluation would.
+ * Synchronous; not for use inside a stream capture.  out (may be NULL, 3
+ * ints): y segment, z segment, CTAs per SM of the flux passes, as in use
+ * after the call.  No counterpart in the reference. */
 AXB_API int axb_batch_autotune(axb_ctx *ctx, axb_batch *batch, int *out, void *stream);
 
 /* ------------------------------------------------------------------------ */
