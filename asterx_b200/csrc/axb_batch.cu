@@ -389,10 +389,12 @@ AXB_API int axb_batch_autotune(axb_ctx *c, axb_batch *B, int *out, void *stream)
     }
     B->seg[d] = best;
   }
-  // the post-step phases take the flux passes' grid size
+  // the light post-step phases take the auxiliaries' grid size.  The recovery
+  // keeps its own: its kernels hold up to 8 CTAs per SM, the flux passes 3, and
+  // at the 4 these often get it ran at half its warps (64 boxes: 824 us at 8,
+  // 1129 us at 4)
   B->ctas[P_SYNC_E] = B->ctas[P_SYNC_P] = B->ctas[P_AUX];
   B->ctas[P_BSTAG] = B->ctas[P_AUX];
-  B->ctas[P_C2P] = B->ctas[P_FLUX_Y];
   if (!rc)
     rc = run_rhs_phases(c, B, s); // leave one consistent RHS evaluation behind
   if (!rc && cudaStreamSynchronize(s) != cudaSuccess)
