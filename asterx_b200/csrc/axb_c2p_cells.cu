@@ -264,7 +264,8 @@ __global__ void __launch_bounds__(128, 8)
     const double det = det3(g);
     const double isg = rsqrt(det);
     const double idet = isg * isg;
-    const double D = c.dens[i] * isg;
+    const double dens = c.dens[i];
+    const double D = dens * isg;
     double S[3], B[3];
     for (int q = 0; q < 3; ++q) {
       S[q] = c.mom[q][i] * isg;
@@ -299,10 +300,18 @@ __global__ void __launch_bounds__(128, 8)
       Ssq = Ssq * (f * f);
     }
     const double BiSi = dot3(S, B);
-    const bool atmosphere = D <= a.atmo.rho_cut;
+    // Near the cut (D is a few ulps off) the densitised variables are compared,
+    // as every other form of the recovery compares them: with atmo_tol zero a
+    // cell set to the atmosphere lies on the cut itself.  One just above it may
+    // fall below after the search, by its rounding: the cascade's.
+    bool atmosphere = D <= a.atmo.rho_cut, at_cut = false;
+    if (fabs(D - a.atmo.rho_cut) <= 1e-14 * a.atmo.rho_cut) {
+      atmosphere = dens <= sqrt(det) * a.atmo.rho_cut;
+      at_cut = !atmosphere;
+    }
     bool common = g.xx > 0.0 && g.xx * g.yy - g.xy * g.xy > 0.0 && det > 0.0 && isfinite(D) &&
                   isfinite(Ssq) && isfinite(Bsq) && isfinite(BiSi) && isfinite(DYe) &&
-                  isfinite(DEnt) && !(Bsq > a.cp.Bsq_lim);
+                  isfinite(DEnt) && !(Bsq > a.cp.Bsq_lim) && !at_cut;
     Prim pv;
     int code = AXB_C2P_PRIME;
     if (common && atmosphere) {

@@ -97,3 +97,25 @@ def test_cells_floors(engine):
     floored = cold & ~fast
     assert np.max(np.abs(got["temperature"][floored] - t_atmo)) <= 1e-15 * t_atmo
     assert np.max(np.abs(got["eps"][floored] - t_atmo / (GAMMA - 1))) <= 1e-14 * t_atmo
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("first", ["noble", "palenzuela"])
+def test_cells_on_the_atmosphere_cut(engine, first):
+    """With atmo_tol = 0 a cell set to the atmosphere (D = sqrt(gamma) rho_atm)
+    lies on the cut itself and is atmosphere again, whatever the metric and
+    whichever scheme is first; one just above it (1e-12) is not."""
+    n = 1000
+    c = _cells(n, seed=11)
+    rho = 3e-9
+    # det gamma as the recovery forms it, so that D is on the cut to the bit
+    xx, xy, xz, yy, yz, zz = (c["g" + k] for k in ("xx", "xy", "xz", "yy", "yz", "zz"))
+    det = xx * (yy * zz - yz * yz) - xy * (xy * zz - yz * xz) + xz * (xy * yz - yy * xz)
+    c["dens"] = np.sqrt(det) * rho
+    c["dens"][::2] *= 1.0 + 1e-12
+    second = "palenzuela" if first == "noble" else "noble"
+    got, _ = _run(engine, c, n, rho_abs_min=rho, atmo_tol=0.0, c2p_prime=first,
+                  c2p_second=second)
+    assert (got["flag"][1::2] == abi.C2P_ATMO).all()
+    assert (got["iters"][1::2] == -1).all() and (got["rho"][1::2] == rho).all()
+    assert (got["flag"][::2] != abi.C2P_ATMO).all()
