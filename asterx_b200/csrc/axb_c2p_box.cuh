@@ -473,9 +473,14 @@ __global__ void __launch_bounds__(128, AXB_C2P_MINB)
 // values fit the registers of NOBLE_MINB CTAs per SM where the whole cascade's
 // spilled; a cell that needs anything else (inside the mask, or a failed Noble search)
 // calls the cascade, out of line and with nothing written.  No queue and no
-// second launch, which small boxes would wait for.  190x131x162 cells 824 ->
-// 590 us (5 CTAs per SM 597, 6: 733, 8: 893), 96^3 195 -> 144 us, 30x39x52 35 ->
-// 15 us.
+// second launch, which small boxes would wait for.  Curl A and recovery of
+// 190x131x162 cells 1192 -> 726 us, 96^3 278 -> 189 us, 20x16x24 40 -> 35 us
+// against the whole cascade in one kernel (CTAs per SM, recovery alone: 4 / 5 /
+// 6 / 8 590 / 597 / 733 / 893 us); with 1 / 10 / 50 % of the cells of 190x131x162
+// failing 9111 / 15490 / 15560 -> 8073 / 12090 / 12103 us, of 128^3 4349 / 6312 /
+// 6319 -> 4289 / 6335 / 6340.  The cascade in one kernel is the faster one where
+// most searches fail: 128^3 at max_iter = 4 (24 % of the cells) 702 -> 905 us, and
+// with half of the cells inside the mask 533 -> 577 us.
 constexpr int NOBLE_MINB = 4;
 template <bool GUESS>
 __device__ __noinline__ void c2p_cascade(const C2PBoxArgs &a, const EosIdeal &eos, int i, int j,
@@ -489,11 +494,11 @@ AXB_D void c2p_noble_body(const C2PBoxArgs &a, const EosIdeal &eos, const uint3 
   int i, j;
   const int k = a.b.ng + bid.z;
   int iters_first = -1;
-  bool failed = false;
+  bool failed = false, rare = false;
   if (a.b.row_ij(a.b.ng, a.b.n[0], a.b.ng, a.b.n[1], bid, i, j)) {
     CellData c;
     c2p_gather(a, eos, i, j, k, c);
-    bool rare = c.alp_avg < a.cp.alp_thresh;
+    rare = c.alp_avg < a.cp.alp_thresh;
     if (!rare) {
       Prim pv;
       int code = AXB_C2P_PRIME;
@@ -519,11 +524,15 @@ AXB_D void c2p_noble_body(const C2PBoxArgs &a, const EosIdeal &eos, const uint3 
       if (!rare)
         c2p_store(a, c.I, code, pv, c.cv);
     }
-    if (rare) {
+    if (rare)
       iters_first = -1;
-      c2p_cascade<GUESS>(a, eos, i, j, k, iters_first, failed);
-    }
   }
+  // cells that left the common path early and late take the cascade together
+  // (one after another: 128^3 with 10 % failing 7980 us, a 64-box level's
+  // recovery 637 instead of 547 us)
+  __syncwarp();
+  if (rare)
+    c2p_cascade<GUESS>(a, eos, i, j, k, iters_first, failed);
   c2p_epilogue(a, s_hist, iters_first, failed);
 }
 template <bool GUESS>

@@ -242,154 +242,177 @@ __global__ void __launch_bounds__(128, AXB_C2P_MINB)
 //
 // With noble_root's cheaper step, 4.0M cells: plain 1156 -> 445 us, learned
 // (recovery alone) 691 -> 297 us.
+//
+// The cascade's 128 registers are not there in 8 CTAs per SM: a cell that needs
+// it costs 1.35 times as long there, and a launch of few blocks waits for one
+// cell.  So a launch that leaves the SMs room takes the form with MINB = 4:
+// 1027 cells, 1 % of them failing, 237 -> 185 us (177 in k_c2p_cells).  In a
+// full launch 8 win: 4.0M cells, 0 / 1 / 10 / 50 % of them failing, 438 / 4717 /
+// 8942 / 9037 us (k_c2p_cells, where every cell waits for its warp's, 1152 /
+// 7307 / 10535 / 10537); over-magnetised instead, 3333 / 9545 / 11579 us (4724 /
+// 10996 / 12836).  Slower than k_c2p_cells are launches where most cells fail
+// their first search: max_iter = 8, with 12 steps a search, 1353 -> 1875 us.
 // ---------------------------------------------------------------------------
+
+// The common path on cell i; false, having written nothing, when it leaves it.
+AXB_D bool c2p_cells_common(const C2PCellsArgs &a, const EosIdeal &eos, const long long i,
+                            int &iters_first) {
+  const axb_cells &c = a.c;
+  const sym3 g{c.g[0][i], c.g[1][i], c.g[2][i], c.g[3][i], c.g[4][i], c.g[5][i]};
+  const double det = det3(g);
+  const double isg = rsqrt(det);
+  const double idet = isg * isg;
+  const double dens = c.dens[i];
+  const double D = dens * isg;
+  double S[3], B[3];
+  for (int q = 0; q < 3; ++q) {
+    S[q] = c.mom[q][i] * isg;
+    B[q] = c.dB[q][i] * isg;
+  }
+  double tau = c.tau[i] * isg;
+  const double DYe = c.DYe[i] * isg;
+  const double DEnt = c.DEnt ? c.DEnt[i] : 0.0;
+  double Bl[3], Sup[3];
+  lower3(g, B, Bl);
+  const double Bsq = dot3(Bl, B);
+  sym3 u; // the inverse metric
+  u.xx = (g.yy * g.zz - g.yz * g.yz) * idet;
+  u.xy = (g.xz * g.yz - g.xy * g.zz) * idet;
+  u.xz = (g.xy * g.yz - g.xz * g.yy) * idet;
+  u.yy = (g.xx * g.zz - g.xz * g.xz) * idet;
+  u.yz = (g.xy * g.xz - g.xx * g.yz) * idet;
+  u.zz = (g.xx * g.yy - g.xy * g.xy) * idet;
+  lower3(u, S, Sup);
+  double Ssq = dot3(S, Sup);
+  // cons_floors_and_ceilings (c2p.hxx:330-369), undensitised
+  const double tau_lim = 0.5 * Bsq;
+  if (tau <= tau_lim)
+    tau = tau_lim;
+  const double slim = D + tau;
+  if (Ssq > slim * slim) {
+    const double f = sqrt(slim * slim / Ssq);
+    for (int q = 0; q < 3; ++q) {
+      S[q] *= f;
+      Sup[q] *= f;
+    }
+    Ssq = Ssq * (f * f);
+  }
+  const double BiSi = dot3(S, B);
+  // Near the cut (D is a few ulps off) the densitised variables are compared,
+  // as every other form of the recovery compares them: with atmo_tol zero a
+  // cell set to the atmosphere lies on the cut itself.  One just above it may
+  // fall below after the search, by its rounding: the cascade's.
+  bool atmosphere = D <= a.atmo.rho_cut, at_cut = false;
+  if (fabs(D - a.atmo.rho_cut) <= 1e-14 * a.atmo.rho_cut) {
+    atmosphere = dens <= sqrt(det) * a.atmo.rho_cut;
+    at_cut = !atmosphere;
+  }
+  bool common = g.xx > 0.0 && g.xx * g.yy - g.xy * g.xy > 0.0 && det > 0.0 && isfinite(D) &&
+                isfinite(Ssq) && isfinite(Bsq) && isfinite(BiSi) && isfinite(DYe) &&
+                isfinite(DEnt) && !(Bsq > a.cp.Bsq_lim) && !at_cut;
+  Prim pv;
+  int code = AXB_C2P_PRIME;
+  if (common && atmosphere) {
+    a.atmo.set(pv);
+    code = AXB_C2P_ATMO;
+  } else if (common) {
+    // start: the learned guess, or the seeds' (Z, v^2)
+    double x0 = -1.0, x1 = -1.0;
+    if (a.use_mlp) {
+      const float2 gs = reinterpret_cast<const float2 *>(c.guess)[i];
+      const double x = gs.x, W = gs.y;
+      x0 = D * x; // Z = rho h W^2 = D (h W)
+      x1 = 1.0 - 1.0 / (W * W);
+      if (!(x0 > 0.0 && x0 < 1e300 && x1 >= 0.0 && x1 < 1.0))
+        x0 = x1 = -1.0;
+    }
+    if (!(x0 >= 0.0)) {
+      double eps = a.atmo.eps, vsq = 0.0;
+      if (c.seed_rho) {
+        double v[3], vl[3];
+        for (int q = 0; q < 3; ++q)
+          v[q] = c.seed_vel[q][i];
+        lower3(g, v, vl);
+        vsq = dot3(vl, v);
+        if (vsq >= 1.0) // limited to v_lim, as con2prim.cxx:168-209
+          vsq = a.cp.v_lim * a.cp.v_lim;
+        eps = fmax(c.seed_eps[i], a.atmo.eps);
+      }
+      // rho = D / W, Z = (rho + eps rho + P) W^2 = D W (1 + eps + P/rho)
+      const double W = rsqrt(1.0 - vsq);
+      x0 = fabs(D * W * (1.0 + eps + eos.gm1 * eps));
+      x1 = vsq;
+    }
+    const NobleRoot r =
+        noble_root<true>(D, tau, Ssq, Bsq, BiSi, a.gamma_noble, a.gfac_over_gamma, a.Zmin,
+                         a.cp.tol, min(a.cp.maxIter, NOBLE_CHEAP_STEPS), x0, x1);
+    common = !r.slow && r.finite;
+    if (common) {
+      // WZ2Prim (c2p_2DNoble.hxx:192-273): W = (1 - v^2)^-1/2, rho = D / W,
+      // eps = (Z / (W^2 rho) - 1) / Gamma = (Z / (W D) - 1) / Gamma
+      const double om = 1.0 - r.vsq;
+      const double W = rsqrt(om);
+      const double iW = om * W;
+      const double iD = 1.0 / D;
+      pv.rho = D * iW;
+      pv.w_lor = W;
+      const double iZZB = 1.0 / (r.Z * (r.Z + Bsq));
+      const double iZB = r.Z * iZZB;
+      for (int q = 0; q < 3; ++q)
+        pv.vel[q] = fma(BiSi * iZZB, B[q], Sup[q] * iZB);
+      pv.eps = fma(r.Z * iW, iD, -1.0) * eos.inv_gamma;
+      pv.Ye = DYe * iD;
+      common = pv.rho > 0.0 && pv.eps > 0.0;
+      if (common) {
+        pv.press = eos.press_from_valid_rho_eps_ye(pv.rho, pv.eps, pv.Ye);
+        pv.temperature = eos.temp_from_valid_rho_eps_ye(pv.rho, pv.eps, pv.Ye);
+        pv.entropy = eos.kappa_from_valid_rho_eps_ye(pv.rho, pv.eps, pv.Ye);
+        iters_first = r.iters;
+        if (pv.rho < a.atmo.rho_cut) {
+          a.atmo.set(pv);
+        } else {
+          Report rep;
+          Cons cv;
+          cv.dens = D;
+          prims_floors(eos, a.cp, a.atmo, pv, cv, g, rep);
+        }
+      }
+    }
+  }
+  if (common)
+    c2p_cells_store(c, i, code, iters_first, false, pv);
+  else
+    iters_first = -1;
+  return common;
+}
+
 __device__ __noinline__ void c2p_cells_cascade(const C2PCellsArgs &a, const EosIdeal &eos,
                                                long long i, int &iters_first, bool &failed) {
   c2p_cells_one(a, eos, i, iters_first, failed);
 }
 
-__global__ void __launch_bounds__(128, 8)
+template <int MINB>
+__global__ void __launch_bounds__(128, MINB)
     k_c2p_cells_noble(const __grid_constant__ C2PCellsArgs a,
                       const __grid_constant__ EosIdeal eos) {
   __shared__ unsigned int s_hist[64];
   for (int q = threadIdx.x; q < 64; q += blockDim.x)
     s_hist[q] = 0;
   __syncthreads();
-  const axb_cells &c = a.c;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   int iters_first = -1;
   bool failed = false;
-  if (i < c.n) {
-    const sym3 g{c.g[0][i], c.g[1][i], c.g[2][i], c.g[3][i], c.g[4][i], c.g[5][i]};
-    const double det = det3(g);
-    const double isg = rsqrt(det);
-    const double idet = isg * isg;
-    const double dens = c.dens[i];
-    const double D = dens * isg;
-    double S[3], B[3];
-    for (int q = 0; q < 3; ++q) {
-      S[q] = c.mom[q][i] * isg;
-      B[q] = c.dB[q][i] * isg;
-    }
-    double tau = c.tau[i] * isg;
-    const double DYe = c.DYe[i] * isg;
-    const double DEnt = c.DEnt ? c.DEnt[i] : 0.0;
-    double Bl[3], Sup[3];
-    lower3(g, B, Bl);
-    const double Bsq = dot3(Bl, B);
-    sym3 u; // the inverse metric
-    u.xx = (g.yy * g.zz - g.yz * g.yz) * idet;
-    u.xy = (g.xz * g.yz - g.xy * g.zz) * idet;
-    u.xz = (g.xy * g.yz - g.xz * g.yy) * idet;
-    u.yy = (g.xx * g.zz - g.xz * g.xz) * idet;
-    u.yz = (g.xy * g.xz - g.xx * g.yz) * idet;
-    u.zz = (g.xx * g.yy - g.xy * g.xy) * idet;
-    lower3(u, S, Sup);
-    double Ssq = dot3(S, Sup);
-    // cons_floors_and_ceilings (c2p.hxx:330-369), undensitised
-    const double tau_lim = 0.5 * Bsq;
-    if (tau <= tau_lim)
-      tau = tau_lim;
-    const double slim = D + tau;
-    if (Ssq > slim * slim) {
-      const double f = sqrt(slim * slim / Ssq);
-      for (int q = 0; q < 3; ++q) {
-        S[q] *= f;
-        Sup[q] *= f;
-      }
-      Ssq = Ssq * (f * f);
-    }
-    const double BiSi = dot3(S, B);
-    // Near the cut (D is a few ulps off) the densitised variables are compared,
-    // as every other form of the recovery compares them: with atmo_tol zero a
-    // cell set to the atmosphere lies on the cut itself.  One just above it may
-    // fall below after the search, by its rounding: the cascade's.
-    bool atmosphere = D <= a.atmo.rho_cut, at_cut = false;
-    if (fabs(D - a.atmo.rho_cut) <= 1e-14 * a.atmo.rho_cut) {
-      atmosphere = dens <= sqrt(det) * a.atmo.rho_cut;
-      at_cut = !atmosphere;
-    }
-    bool common = g.xx > 0.0 && g.xx * g.yy - g.xy * g.xy > 0.0 && det > 0.0 && isfinite(D) &&
-                  isfinite(Ssq) && isfinite(Bsq) && isfinite(BiSi) && isfinite(DYe) &&
-                  isfinite(DEnt) && !(Bsq > a.cp.Bsq_lim) && !at_cut;
-    Prim pv;
-    int code = AXB_C2P_PRIME;
-    if (common && atmosphere) {
-      a.atmo.set(pv);
-      code = AXB_C2P_ATMO;
-    } else if (common) {
-      // start: the learned guess, or the seeds' (Z, v^2)
-      double x0 = -1.0, x1 = -1.0;
-      if (a.use_mlp) {
-        const float2 gs = reinterpret_cast<const float2 *>(c.guess)[i];
-        const double x = gs.x, W = gs.y;
-        x0 = D * x; // Z = rho h W^2 = D (h W)
-        x1 = 1.0 - 1.0 / (W * W);
-        if (!(x0 > 0.0 && x0 < 1e300 && x1 >= 0.0 && x1 < 1.0))
-          x0 = x1 = -1.0;
-      }
-      if (!(x0 >= 0.0)) {
-        double eps = a.atmo.eps, vsq = 0.0;
-        if (c.seed_rho) {
-          double v[3], vl[3];
-          for (int q = 0; q < 3; ++q)
-            v[q] = c.seed_vel[q][i];
-          lower3(g, v, vl);
-          vsq = dot3(vl, v);
-          if (vsq >= 1.0) // limited to v_lim, as con2prim.cxx:168-209
-            vsq = a.cp.v_lim * a.cp.v_lim;
-          eps = fmax(c.seed_eps[i], a.atmo.eps);
-        }
-        // rho = D / W, Z = (rho + eps rho + P) W^2 = D W (1 + eps + P/rho)
-        const double W = rsqrt(1.0 - vsq);
-        x0 = fabs(D * W * (1.0 + eps + eos.gm1 * eps));
-        x1 = vsq;
-      }
-      const NobleRoot r =
-          noble_root<true>(D, tau, Ssq, Bsq, BiSi, a.gamma_noble, a.gfac_over_gamma, a.Zmin,
-                           a.cp.tol, a.cp.maxIter, x0, x1);
-      common = !r.slow && r.finite;
-      if (common) {
-        // WZ2Prim (c2p_2DNoble.hxx:192-273): W = (1 - v^2)^-1/2, rho = D / W,
-        // eps = (Z / (W^2 rho) - 1) / Gamma = (Z / (W D) - 1) / Gamma
-        const double om = 1.0 - r.vsq;
-        const double W = rsqrt(om);
-        const double iW = om * W;
-        const double iD = 1.0 / D;
-        pv.rho = D * iW;
-        pv.w_lor = W;
-        const double iZZB = 1.0 / (r.Z * (r.Z + Bsq));
-        const double iZB = r.Z * iZZB;
-        for (int q = 0; q < 3; ++q)
-          pv.vel[q] = fma(BiSi * iZZB, B[q], Sup[q] * iZB);
-        pv.eps = fma(r.Z * iW, iD, -1.0) * eos.inv_gamma;
-        pv.Ye = DYe * iD;
-        common = pv.rho > 0.0 && pv.eps > 0.0;
-        if (common) {
-          pv.press = eos.press_from_valid_rho_eps_ye(pv.rho, pv.eps, pv.Ye);
-          pv.temperature = eos.temp_from_valid_rho_eps_ye(pv.rho, pv.eps, pv.Ye);
-          pv.entropy = eos.kappa_from_valid_rho_eps_ye(pv.rho, pv.eps, pv.Ye);
-          iters_first = r.iters;
-          if (pv.rho < a.atmo.rho_cut) {
-            a.atmo.set(pv);
-          } else {
-            Report rep;
-            Cons cv;
-            cv.dens = D;
-            prims_floors(eos, a.cp, a.atmo, pv, cv, g, rep);
-          }
-        }
-      }
-    }
-    if (common) {
-      c2p_cells_store(c, i, code, iters_first, false, pv);
-    } else {
-      iters_first = -1;
-      c2p_cells_cascade(a, eos, i, iters_first, failed);
-    }
-  }
+  const bool rest = i < a.c.n && !c2p_cells_common(a, eos, i, iters_first);
+  // cells that left the common path early and late take the cascade together
+  // (one after another, 10 % over-magnetised cells of 1027 took 391 us, not 220)
+  __syncwarp();
+  if (rest)
+    c2p_cells_cascade(a, eos, i, iters_first, failed);
   c2p_cells_epilogue(a, s_hist, iters_first, failed);
 }
+// cells from which 8 CTAs per SM win: 100003 / 200000 / 400000 cells 30 / 43 /
+// 90 us at 4 and 31 / 46 / 87 at 8 CTAs per SM
+constexpr long long CELLS_FULL = 1 << 18;
 } // namespace axb
 
 AXB_API int axb_c2p_cells(axb_ctx *ctx, const axb_cells *cells, const axb_params *p,
@@ -478,8 +501,10 @@ AXB_API int axb_c2p_cells(axb_ctx *ctx, const axb_cells *cells, const axb_params
   axb_mark(ctx, AXB_R_C2P_CELLS, s, true);
   if (eos->kind == 1)
     k_c2p_cells<<<(unsigned)blocks, 128, 0, s>>>(a, tab_for_launch(*eos, a.status));
+  else if (a.c2p_prime == AXB_C2P_NOBLE && !a.cp.use_zprim && cells->n < CELLS_FULL)
+    k_c2p_cells_noble<4><<<(unsigned)blocks, 128, 0, s>>>(a, eos->ideal);
   else if (a.c2p_prime == AXB_C2P_NOBLE && !a.cp.use_zprim)
-    k_c2p_cells_noble<<<(unsigned)blocks, 128, 0, s>>>(a, eos->ideal);
+    k_c2p_cells_noble<8><<<(unsigned)blocks, 128, 0, s>>>(a, eos->ideal);
   else
     k_c2p_cells<<<(unsigned)blocks, 128, 0, s>>>(a, eos->ideal);
   axb_mark(ctx, AXB_R_C2P_CELLS, s, false);

@@ -119,3 +119,26 @@ def test_cells_on_the_atmosphere_cut(engine, first):
     assert (got["flag"][1::2] == abi.C2P_ATMO).all()
     assert (got["iters"][1::2] == -1).all() and (got["rho"][1::2] == rho).all()
     assert (got["flag"][::2] != abi.C2P_ATMO).all()
+
+
+@pytest.mark.gpu
+def test_small_and_large_launches_agree(engine):
+    """A launch that fills the GPU (8 CTAs per SM) and launches of few blocks
+    (the registers the cascade wants) give every cell the same bits, on the
+    common path and off it; the failure count is that of the flags."""
+    n = (1 << 18) + 77
+    c = _cells(n, seed=21)
+    u = np.random.default_rng(4).uniform(size=n)
+    sq = c["dens"] / (c["rho"] * c["W"])
+    c["tau"] = np.where(u < 0.01, np.nan, c["tau"])
+    c["dBx"] = np.where((u > 0.01) & (u < 0.03), c["dBx"] * 1e9, c["dBx"])
+    c["dens"] = np.where((u > 0.03) & (u < 0.04), sq * 1e-15, c["dens"])
+    c["gxx"] = np.where((u > 0.04) & (u < 0.05), -1.0, c["gxx"])
+    got, st = _run(engine, c, n, B_lim=1e8)
+    flags = np.bincount(got["flag"].astype(int), minlength=7)
+    assert flags[abi.C2P_FAIL] == st["c2p_fail"] > 0 and flags[abi.C2P_ATMO] > 0
+    assert flags[abi.C2P_PRIME] > 0.9 * n
+    for lo, hi in ((0, 1), (1000, 3000), (n // 2, n // 2 + 5000), (n - 100, n)):
+        part, _ = _run(engine, {k: v[lo:hi] for k, v in c.items()}, hi - lo, B_lim=1e8)
+        for k, v in part.items():
+            assert np.array_equal(v, got[k][lo:hi], equal_nan=True), (k, lo)
