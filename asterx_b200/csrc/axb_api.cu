@@ -821,11 +821,8 @@ int launch_rhs_misc(int which, const RhsArgs &a, cudaStream_t s) {
       ap.b.packed = 1;
       grid = dim3(unsigned(plane), 1, 1);
     }
-    const int n = b.n[2];
-    const int seg = split_steps(n, double(SOURCES_MINB) * sm_count(), SOURCES_START, [&](int q) {
-      return (long long)grid.x * grid.y * ((n + q - 1) / q);
-    });
-    grid.z = (n + seg - 1) / seg;
+    const int seg = sources_steps(b.n[2], (long long)grid.x * grid.y, sm_count());
+    grid.z = (b.n[2] + seg - 1) / seg;
     if (which == 0)
       k_sources_column<2><<<grid, T, 0, s>>>(ap, seg);
     else

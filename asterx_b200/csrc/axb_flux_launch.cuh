@@ -25,26 +25,18 @@ int launch_flux_pass_uct(int dir, const RhsArgs &a, const EOS &eos, cudaStream_t
     k_flux_x<RECON, EOS, UCT><<<(unsigned)blocks, 128, 0, s>>>(a, eos);
     return cudaGetLastError() == cudaSuccess ? AXB_OK : AXB_ERR_CUDA;
   }
-  const int T0 = 0, T1 = dir == 2 ? 1 : 2, n = b.n[dir];
-  const double slots = double(FLUX_MINB) * sm_count();
-  const dim3 block(FLUX_T);
   // The threads walk the transverse plane [ng-1, ng+n]^2 row after row (as in
   // the batched kernels), so the 2 extra columns of the plane do not leave most
   // of a warp idle.  (Blocks of 32 columns x 4 rows, which MP5 was faster on
   // while its stencils came through L1: 128^3 substep 3.19 ms, 2.88 so; 96^3
   // tabulated RHS 3.49 ms, 2.48 so.)
-  RhsArgs ap = a;
-  ap.b.packed = 1;
-  const long long plane = (long long)(b.n[T0] + 2 * a.text) * (b.n[T1] + 2 * a.text);
-  dim3 grid(unsigned((plane + FLUX_T - 1) / FLUX_T), 1, 1);
-  const int seglen = split_steps(n, slots, FLUX_START, [&](int seg) {
-    return (long long)grid.x * ((n + seg - 1) / seg);
-  });
-  grid.z = (n + seglen - 1) / seglen;
+  const int seglen = flux_steps(b, dir, a.text, sm_count());
+  const dim3 grid(unsigned(flux_plane_blocks(b, dir, a.text)), 1,
+                  (b.n[dir] + seglen - 1) / seglen);
   if (dir == 1)
-    launch_pass(k_flux_pass<1, RECON, EOS, UCT>, grid, block, s, ap, eos, seglen);
+    launch_pass(k_flux_pass<1, RECON, EOS, UCT>, grid, dim3(FLUX_T), s, a, eos, seglen);
   else
-    launch_pass(k_flux_pass<2, RECON, EOS, UCT>, grid, block, s, ap, eos, seglen);
+    launch_pass(k_flux_pass<2, RECON, EOS, UCT>, grid, dim3(FLUX_T), s, a, eos, seglen);
   return cudaGetLastError() == cudaSuccess ? AXB_OK : AXB_ERR_CUDA;
 }
 

@@ -1,6 +1,7 @@
 // RHS kernels (see axb_rhs.cuh for the overview).
 #pragma once
 
+#include "axb_internal.hxx"
 #include "axb_rhs.cuh"
 
 namespace axb {
@@ -360,6 +361,18 @@ AXB_D void flux_pass_body(const RhsArgs &a, const EOS &eos, const int &seglen, c
     }
   }
   flux_status(a, smax, bad, bad_rhs);
+}
+// blocks that cover the transverse plane of a y or z pass once, and the steps of
+// a box's pencils in it
+inline long long flux_plane_blocks(const BoxDev &b, int dir, int te) {
+  const long long plane = (long long)(b.n[0] + 2 * te) * (b.n[dir == 2 ? 1 : 2] + 2 * te);
+  return (plane + FLUX_T - 1) / FLUX_T;
+}
+inline int flux_steps(const BoxDev &b, int dir, int te, int sms) {
+  const long long plane = flux_plane_blocks(b, dir, te);
+  const int n = b.n[dir];
+  return split_steps(n, double(FLUX_MINB) * sms, FLUX_START,
+                     [&](int seg) { return plane * ((n + seg - 1) / seg); });
 }
 template <int DIR, int RECON, class EOS, bool UCT = false>
 __global__ void __launch_bounds__(FLUX_T, FLUX_MINB)

@@ -284,6 +284,12 @@ AXB_D void sources_column(const RhsArgs &a, const uint3 bid, const int seg) {
   }
 }
 
+// cells of a column of the sources of a box whose (i, j) plane takes `plane`
+// blocks
+inline int sources_steps(int n, long long plane, int sms) {
+  return split_steps(n, double(SOURCES_MINB) * sms, SOURCES_START,
+                     [&](int seg) { return plane * ((n + seg - 1) / seg); });
+}
 template <int FD>
 __global__ void __launch_bounds__(128, SOURCES_MINB)
     k_sources_column(const RhsArgs a, const int seg) {

@@ -1,6 +1,6 @@
 """The RHS group at the edges of the flux passes' tiles (30-cell chunks along
-x, 128 pencils of the transverse plane, pencil segments) and of the sources'
-z columns, against the restated reference: largest error over the largest
+x, 128 pencils of the transverse plane, pencil segments of one step and of
+several) and of the sources' z columns, against the restated reference: largest error over the largest
 value <= 1e-12, as the RHS parity tests take it (both sides evaluate the same
 formulas in FP64; multiply-add contraction and shared reciprocals move the
 last ulps)."""
@@ -13,6 +13,11 @@ from oracle.oracle import restatement
 from tests.helpers import errors, full_fields, interior
 
 SIZES = [(3, 4, 5), (29, 4, 3), (30, 5, 33), (31, 18, 4), (64, 3, 35), (5, 66, 17)]
+# boxes whose pencils and columns take 6 or 7 steps, the last one fewer, on a
+# GPU of SMS multiprocessors (test_steps.py holds the split to that; the boxes
+# above take one step a thread)
+LONG = [(61, 130, 37)]
+SMS = 148
 
 
 def _box(n, seed):
@@ -31,8 +36,11 @@ def _box(n, seed):
 @pytest.mark.gpu
 @pytest.mark.parametrize("recon,flux,order", [("wenoz", "hlle", 2), ("mp5", "lxf", 4),
                                               ("ppm", "hlle", 2), ("minmod", "hlle", 4)])
-@pytest.mark.parametrize("n", SIZES)
+@pytest.mark.parametrize("n", SIZES + LONG)
 def test_rhs_tiles(engine, n, recon, flux, order):
+    if n in LONG:
+        props = engine.torch.cuda.get_device_properties(engine.device)
+        assert props.multi_processor_count == SMS
     L, f = _box(n, seed=sum(n))
     p = abi.default_params(reconstruction_method=recon, flux_type=flux,
                            local_spatial_order=order)
