@@ -126,14 +126,18 @@ def peak_hbm():
         return 6650.0, "fallback"
 
 
-def traffic_table():
-    """Per-launch DRAM bytes from the committed ncu summaries (profiles/)."""
+def kernel_traffic(region, recon, n):
+    """Per-launch DRAM bytes of a kernel and where they come from: the committed
+    ncu captures of 128^3 boxes (profiles/), scaled by the zones for others."""
     p = os.path.join(REPO, "profiles", "traffic.json")
     try:
         with open(p) as fh:
-            return json.load(fh)
+            captured = json.load(fh)[f"{region}:{recon}:128"]
     except Exception:
-        return {}
+        return None, None
+    if n == 128:
+        return captured, "ncu capture at 128^3"
+    return captured * (n / 128) ** 3, f"ncu capture at 128^3 x ({n}/128)^3"
 
 
 class ClockSampler:
@@ -478,7 +482,7 @@ def ours(args):
     alg_bytes = ALG_DOUBLES[dom] * 8 * zones
     achieved = alg_bytes / avg_launch_s / 1e9
     peak, peak_kind = peak_hbm()
-    traffic = traffic_table().get(f"{dom}:{args.recon}:{args.n}")
+    traffic, traffic_from = (None, None) if tab else kernel_traffic(dom, args.recon, args.n)
     substep_gbs = SUBSTEP_BYTES * zones / (ms / args.steps / 1e3) / 1e9
 
     # end to end through the C ABI from pinned host memory: every step copies
@@ -550,6 +554,7 @@ def ours(args):
             "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved,
                          "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,
+                         "traffic_from": traffic_from,
                          "alg_bytes_per_launch": alg_bytes,
                          "avg_launch_ms": avg_launch_s * 1e3,
                          "substep": {"alg_bytes_per_zone": SUBSTEP_BYTES,
