@@ -25,10 +25,11 @@ FLAGS = ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr",
 # Per-file flags.  The recovery is compiled without multiply-add contraction:
 # every FP64 operation is rounded on its own, as written, so the same cell
 # gives the same bits whichever kernel (single box, fast pass, deferred
-# pass, batched level) inlines the recovery -- contraction choices depend on
-# the surrounding code, and the Brent bracket amplifies a last-bit
+# pass, batched level) inlines the same expressions -- contraction choices
+# depend on the surrounding code, and the Brent bracket amplifies a last-bit
 # difference to the root-finder tolerance.  It also follows the per-operation
-# rounding of the reference's CPU build.
+# rounding of the reference's CPU build.  (The kernels for Noble first on the
+# ideal gas write their multiply-adds out.)
 # The recovery is split over three translation units (single box, batched,
 # independent cells) that share axb_c2p_box.cuh, so they compile in parallel.
 # The stress-energy tensor and the regrid error follow the reference's

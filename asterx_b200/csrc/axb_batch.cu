@@ -5,8 +5,9 @@
 // every level), so a level of 512 small boxes costs ~5600 kernel launches per
 // substep.  Here every phase of the substep is ONE persistent launch over the
 // tiles of all boxes (axb_batch.cuh), the per-box argument blocks live in
-// device memory, and the whole substep (11 launches plus one memset of the
-// work counters) is stream-ordered and allocation-free, so a caller can
+// device memory, and the whole substep (11 launches and a memset of the work
+// counters; with Palenzuela first one more of each, for the queue of deferred
+// cells) is stream-ordered and allocation-free, so a caller can
 // capture it in a CUDA graph.  The pencil segments of the y and z flux passes
 // follow from the level's size; the autotuner checks them, and the number of
 // resident CTAs per SM of the persistent grids, by timing the batch's own boxes.

@@ -3,12 +3,14 @@
 // A batched launch runs one kernel body over the tiles (CTA-sized work
 // items) of every box of a batch.  The tiles of box b are items
 // [prefix[b], prefix[b+1]) of a flat list; the tile's block index inside
-// its box is unflattened from the box's own grid, so every body sees exactly
-// the block indices its single-box launch would give it and the results are
-// bit-identical to one launch per box.  The grid is persistent: each CTA
-// draws chunks of items from an atomic work counter, and copies the per-box
-// argument block
-// into shared memory when it moves on to the next box.
+// its box is unflattened from the box's own grid.  The bodies are those of the
+// single-box launches; the level's grids may pack planes and split pencils
+// otherwise (its tiles are counted over all boxes), and the compiler contracts
+// the flux kernels' multiply-adds kernel by kernel, so a level's results are
+// those of one launch per box to the last ulps of the RHS.  The grid is
+// persistent: each CTA draws chunks of items from an atomic work counter, and
+// copies the per-box argument block into shared memory when it moves on to the
+// next box.
 #pragma once
 
 #include <type_traits>

@@ -385,13 +385,14 @@ AXB_HD void set_E(Prim &pv, const sym3 &gup) {
 // A cheap search that does not converge writes nothing: the cell goes through
 // the cascade, whose expressions decide.  One that converges is taken, also
 // where the reference's would have stopped at max_iter.  Flags that differ, of
-// 4.0M independent cells each, all of them recovered instead of failed: none
-// with eps >= 1e-6, b^2/rho <= 100 and W <= 50 at tol = 1e-10 (one at 1e-12), nor
-// in boxes of 1.4M cells at W <= 30 and max_iter from 4 on; in cold flow (eps
-// to 1e-9) with b^2/rho to 1e4, where the last steps are noise, 1.4e-4 at
-// tol = 1e-10 and 3e-3 at 1e-12 with max_iter = 30 (1e-5 and 1e-3 with 100).  A
-// cheap search stops after NOBLE_CHEAP_STEPS: 44 was the most that one of 2M
-// cells of the first range took, beyond it is noise.
+// 4.0M independent cells each, all of them recovered instead of failed: with
+// eps >= 1e-6, b^2/rho <= 100 and W <= 50 none at tol = 1e-10 and one at 1e-12
+// (max_iter 30 or 100; up to one and 40 at max_iter = 10, where the mean search
+// takes 12), and none in boxes of 1.4M cells at W <= 30 and max_iter from 4 on; in
+// cold flow (eps to 1e-9) with b^2/rho to 1e4, where the last steps are noise,
+// 1.4e-4 at tol = 1e-10 and 3e-3 at 1e-12 with max_iter = 30 (1e-5 and 1e-3 with
+// 100).  A cheap search stops after NOBLE_CHEAP_STEPS: 58 was the most that one of
+// 6.7e7 cells of the first range took, beyond it is noise.
 constexpr int NOBLE_CHEAP_STEPS = 64;
 struct NobleRoot {
   double Z, vsq;

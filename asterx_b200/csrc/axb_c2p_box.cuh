@@ -6,8 +6,12 @@
 // ones (axb_c2p_batch.cu) and the independent-cell recovery
 // (axb_c2p_cells.cu); each translation unit instantiates the kernels it
 // launches.  Every file that includes this is compiled without multiply-add
-// contraction (asterx_b200/build.py), so all kernels give a cell the same
-// bits.
+// contraction (asterx_b200/build.py), so the kernels that run the same
+// expressions give a cell the same bits: the fast pass, the deferred pass and
+// the whole cascade, on one box and on a level.  The kernels for Noble first on
+// the ideal gas take another form of its Newton step (noble_root's CHEAP, and the
+// independent cells' undensitised variables) and agree with the cascade to the
+// search's tolerance.
 #pragma once
 
 #include <algorithm>

@@ -221,13 +221,14 @@ AXB_D void cp_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory")
 // copied asynchronously into the slot of the row just used while the face is
 // computed, and a step reads 9 doubles from memory for its stencils instead of
 // 45.  With the carried upper values and fluxes that is 488 bytes a thread;
-// three CTAs per SM fit, whose 168 registers hold both face states without
-// spills (four at 128 registers spilled, and kept the left state in shared
-// memory).  256^3 WENO-Z: y 3.55 -> 2.87 ms, z 3.80 -> 3.09 ms (beside the
+// three CTAs per SM fit, whose 168 registers hold both face states: without
+// spills for the ideal gas on one box, with 0.1 KB (stores; 0.14 KB loads) in a
+// level's kernels, whose draw of tiles stays live, and 0.2 (0.3) KB on a table
+// (four CTAs at 128 registers spilled, and kept the left state in shared memory).  256^3 WENO-Z: y 3.55 -> 2.87 ms, z 3.80 -> 3.09 ms (beside the
 // sources; with fold_divergence's loads ahead of its stores, and the z pass's
-// in two batches from U prefetched, 2.52 and 2.49 ms).  Not kept: a four-slot ring with the last row loaded directly at
-// four CTAs (3.05 / 3.31 ms) or three (2.95 / 3.09); seven 64-thread CTAs at
-// 128 registers (3.39 / 3.66).
+// in two batches from U prefetched, 2.52 and 2.49 ms).  Not kept: a four-slot
+// ring with the last row loaded directly at four CTAs (3.05 / 3.31 ms) or three
+// (2.95 / 3.09); seven 64-thread CTAs at 128 registers (3.39 / 3.66).
 // Transverse range: cells [ng-1, ng+n] (one ghost layer each side, needed
 // by the edge electric field); faces along DIR: [ng, ng+n].
 // ---------------------------------------------------------------------------

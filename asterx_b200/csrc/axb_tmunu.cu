@@ -11,8 +11,9 @@
 //                          estimate_error.cxx:70-144) with the indicators of
 //                          AsterX/src/estimate_error.hxx:14-86
 //
-// k_tmunu2 and k_regrid_error are HBM-bound point loops (one thread per point,
-// rows of 128 along x, neighbours from L1/L2).  This file is compiled without multiply-add
+// k_tmunu2 (a plane's vertices row after row, 72 loads a vertex through L1,
+// which bounds it) and k_regrid_error (rows of 128 along x, HBM) run one thread
+// per point; k_tmunu4 runs tiles.  This file is compiled without multiply-add
 // contraction and keeps the reference's operation order (sums from left to
 // right, products left-associated as written), so the results are the
 // reference's bits: IEEE division and square root round the same on both.

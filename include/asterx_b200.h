@@ -437,8 +437,10 @@ AXB_API int axb_substep(axb_ctx *ctx, const axb_box *box,
 /* A level of boxes advanced together.  CarpetX runs each scheduled routine
  * of AsterX_RHSGroup and AsterX_Con2PrimGroup (AsterX/schedule.ccl:119-228)
  * as one loop launch per box; a batch runs each phase of the substep as ONE
- * persistent launch over the tiles of all its boxes, with results
- * bit-identical to axb_substep on every box.  axb_batch_create checks every
+ * persistent launch over the tiles of all its boxes.  The results are those
+ * of axb_substep on every box to the last ulps of the RHS (multiply-adds are
+ * contracted kernel by kernel), which a recovery carries to at most its
+ * tolerance.  axb_batch_create checks every
  * box as axb_rhs_group / axb_con2prim_group would, copies the per-box
  * argument blocks and tile tables to the device (its only allocations), and
  * keeps `eos` by reference: it must outlive the batch.  Field pointers are
@@ -451,7 +453,8 @@ AXB_API int axb_batch_create(axb_ctx *ctx, int nbox, const axb_box *boxes,
 AXB_API int axb_batch_destroy(axb_batch *batch);
 
 /* One RK substep of every box (axb_substep semantics), as 11 stream-ordered
- * launches and one memset, allocation-free: a caller may capture it in a
+ * launches and one memset (one more of each with Palenzuela first),
+ * allocation-free: a caller may capture it in a
  * CUDA graph. */
 AXB_API int axb_batch_substep(axb_ctx *ctx, axb_batch *batch, double alpha,
                               double beta, double gamma, double dt, int periodic,
