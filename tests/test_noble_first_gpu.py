@@ -1,9 +1,10 @@
 """The box recovery with Noble first on the ideal gas, alone and as the boxes of
 a level: its own kernels, whose common path leaves cells inside the mask,
-non-finite ones and those of a failed search to the whole cascade.  Against the restated reference on rows at the edges of a block: flags
-identical, failures counted, values within 1e-9 of their largest value where
-a search stops at 1e-12 of its unknown (the recovery amplifies that by at most
-about 1e3 for W <= 3, b^2/rho <= 0.3 and eps >= 0.1)."""
+non-finite ones and those of a failed search to the whole cascade.  Against the
+restated reference on rows at the edges of a block: flags identical, failures
+counted, values within 1e-9 of their largest value where a search stops at 1e-12
+of its unknown (the recovery amplifies that by at most about 1e3 for W <= 3,
+b^2/rho <= 0.3 and eps >= 0.1)."""
 import numpy as np
 import pytest
 
